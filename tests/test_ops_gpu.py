@@ -31,6 +31,22 @@ def test_rmsnorm_fwd_bwd(rows, D):
   assert (ds - dsr).abs().max() <= 2e-2 * max(1.0, dsr.abs().max().item())
 
 
+@pytest.mark.parametrize("rows,D", [(1, 8), (7, 128), (31, 512), (4800, 128), (33, 520), (700, 1032), (1300, 4096)])
+def test_rmsnorm_scale_gradient_adds_every_row_once(rows, D):
+  """Row counts around the blocks of the first pass and the row lanes of the second; the gradient joins what is there already. Any order of an
+  fp32 sum of n products is within (n + 4) 2**-24 of the sum of their absolute values (two roundings in each product, one for rstd)."""
+  E = _E()
+  x, dy = (torch.randn(rows, D, device="cuda").bfloat16() for _ in range(2))
+  scale = torch.ones(D, device="cuda").bfloat16()
+  y, dx, rstd = torch.empty_like(x), torch.empty_like(x), torch.empty(rows, device="cuda")
+  E.rmsnorm_fwd(x, scale, 1e-5, 0.0, y, rstd)
+  ds = torch.full((D,), 3.0, device="cuda")
+  E.rmsnorm_bwd(dy, x, scale, rstd, 0.0, dx, ds)
+  terms = dy.double() * x.double() * rstd.double()[:, None]
+  bound = (terms.abs().sum(0) + 3.0) * (rows + 4) * 2.0 ** -24
+  assert bool(((ds.double() - 3.0 - terms.sum(0)).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 def test_rope_roundtrip_and_reference(interleaved):
   E = _E()
