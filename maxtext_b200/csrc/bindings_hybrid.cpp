@@ -156,7 +156,7 @@ void check_cache(const Tensor& k, const Tensor& v, const Tensor& like, int64_t D
 void qkv_prep(const Tensor& q, const Tensor& k, const Tensor& v, int64_t D, int64_t Dv, const Tensor& pos, const OptTensor& inv_ts, int64_t rot, double eps,
               Tensor& qp, const OptTensor& kp, const OptTensor& vp, Tensor& kc, Tensor& vc, const Tensor& slots, const Tensor& lengths,
               const OptTensor& new_lens, const OptTensor& bq, const OptTensor& bk, const OptTensor& bv, const OptTensor& wq, const OptTensor& wk, bool paired,
-              int64_t maps, double temp_coef, double temp_every, const OptTensor& talk) {
+              int64_t maps, double temp_coef, double temp_every, const OptTensor& talk, bool steps, double q_mult) {
   const bool f = f32(q);
   TORCH_CHECK(qp.dim() == 3 && rot % 2 == 0 && rot >= 0 && rot <= D && bool(inv_ts) == (rot > 0) && maps >= 1 && qp.size(1) % maps == 0);
   const int64_t N = q.size(0), H = qp.size(1) / maps, dq = qp.size(2), B = slots.numel();
@@ -182,6 +182,8 @@ void qkv_prep(const Tensor& q, const Tensor& k, const Tensor& v, int64_t D, int6
   a.inv_ts = inv_ts ? inv_ts->data_ptr<float>() : nullptr;
   a.rot = (int)rot; a.paired = paired;
   a.eps = (float)eps; a.temp_coef = (float)temp_coef; a.temp_every = (float)temp_every;
+  TORCH_CHECK(steps || q_mult == 1.0);
+  a.steps = steps; a.q_mult = (float)q_mult;
   a.S = (int)(N / B);
   a.talk = same(talk, q, H * H, "mixing matrix");
   a.qp = qp.data_ptr(); a.kp = kp ? kp->data_ptr() : nullptr; a.vp = vp ? vp->data_ptr() : nullptr;
@@ -379,7 +381,8 @@ void register_hybrid(pybind11::module_& m) {
   const auto none = pybind11::none();
   m.def("qkv_prep", &qkv_prep, arg("q"), arg("k"), arg("v"), arg("D"), arg("Dv"), arg("pos"), arg("inv_ts"), arg("rot"), arg("eps"), arg("qp"), arg("kp"),
         arg("vp"), arg("kc"), arg("vc"), arg("slots"), arg("lengths"), arg("new_lens"), arg("bq") = none, arg("bk") = none, arg("bv") = none, arg("wq") = none,
-        arg("wk") = none, arg("paired") = false, arg("maps") = 1, arg("temp_coef") = 0.0, arg("temp_every") = 0.0, arg("talk") = none);
+        arg("wk") = none, arg("paired") = false, arg("maps") = 1, arg("temp_coef") = 0.0, arg("temp_every") = 0.0, arg("talk") = none, arg("steps") = false,
+        arg("q_mult") = 1.0);
   m.def("cached_decode_splits", &cached_decode_splits);
   m.def("cached_decode", &cached_decode, arg("q"), arg("k"), arg("v"), arg("slots"), arg("lengths"), arg("scale"), arg("cap"), arg("window"), arg("sinks"),
         arg("gate"), arg("splits"), arg("part"), arg("ml"), arg("out"), arg("chunk") = 0, arg("per_head") = false, arg("lam") = std::vector<Tensor>{},

@@ -69,6 +69,14 @@ __device__ __forceinline__ void load_talk(const PrepArgs& a, float* st) {
   }
 }
 
+// what a value is after a trip through memory
+template <typename T>
+__device__ __forceinline__ float stored(float x) { return to_f(from_f<T>(x)); }
+
+// the two lanes of a rotated pair; written out so that every kernel that turns a pair rounds alike
+__device__ __forceinline__ float turn_low(float a, float b, float2 c) { return __fmaf_rn(a, c.x, -__fmul_rn(b, c.y)); }
+__device__ __forceinline__ float turn_high(float a, float b, float2 c) { return __fmaf_rn(a, c.y, __fmul_rn(b, c.x)); }
+
 // floats of shared memory in front of the mixing operands (a multiple of four)
 __host__ __device__ __forceinline__ int angle_floats(int rot) { return (rot + 2 + 3) / 4 * 4; }
 
@@ -99,7 +107,7 @@ qkv_prep_kernel(const PrepArgs a) {
       float y[VEC];
       load_vec<VEC>(bias + (long)head * D + e0, y);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) x[e] += y[e];
+      for (int e = 0; e < VEC; ++e) x[e] = a.steps ? stored<T>(x[e] + y[e]) : x[e] + y[e];
     }
   };
   float rstd_q = 1.f, rstd_k = 1.f;
@@ -155,7 +163,11 @@ qkv_prep_kernel(const PrepArgs a) {
       float g[VEC];
       if (w) load_vec<VEC>(w + e0, g);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) y[e] *= w ? r * g[e] : r;
+      for (int e = 0; e < VEC; ++e) y[e] = a.steps && w ? stored<T>(y[e] * r) * g[e] : y[e] * (w ? r * g[e] : r);
+      if (a.steps) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) y[e] = stored<T>(y[e]);
+      }
     };
 #pragma unroll
     for (int it = 0; it < ITER; ++it) {
@@ -172,27 +184,27 @@ qkv_prep_kernel(const PrepArgs a) {
 #pragma unroll
           for (int e = 0; e < VEC; ++e) {
             const float2 c = cs[(low ? e0 : e0 - half) + e];
-            x[it][e] = x[it][e] * c.x + (low ? -y[e] : y[e]) * c.y;
+            x[it][e] = low ? turn_low(x[it][e], y[e], c) : turn_high(y[e], x[it][e], c);
           }
         } else if constexpr (VEC > 1) {
 #pragma unroll
           for (int e = 0; e < VEC; e += 2) {
             const float2 c = cs[(e0 + e) / 2];
             const float u = x[it][e], v = x[it][e + 1];
-            x[it][e] = u * c.x - v * c.y;
-            x[it][e + 1] = v * c.x + u * c.y;
+            x[it][e] = turn_low(u, v, c);
+            x[it][e + 1] = turn_high(u, v, c);
           }
         } else {
           float y[VEC];
           raw(key, head, e0 ^ 1, y);
           scaled(e0 ^ 1, y);
           const float2 c = cs[e0 / 2];
-          x[it][0] = x[it][0] * c.x + (e0 & 1 ? y[0] : -y[0]) * c.y;
+          x[it][0] = e0 & 1 ? turn_high(y[0], x[it][0], c) : turn_low(x[it][0], y[0], c);
         }
       }
       if (!key) {
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) x[it][e] *= warm;
+        for (int e = 0; e < VEC; ++e) x[it][e] = (a.steps ? stored<T>(stored<T>(x[it][e]) * a.q_mult) : x[it][e]) * warm;
       }
     }
     const int m = head % a.maps;                            // this map's lanes of the head
@@ -264,7 +276,7 @@ qkv_prep_wide_kernel(const PrepArgs a) {
         float y[VEC];
         load_vec<VEC>(bias + (long)head * D + e0, y);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) x[e] += y[e];
+        for (int e = 0; e < VEC; ++e) x[e] = a.steps ? stored<T>(x[e] + y[e]) : x[e] + y[e];
       }
     } else {
 #pragma unroll
@@ -341,7 +353,7 @@ qkv_prep_wide_kernel(const PrepArgs a) {
       float g[VEC];
       load_vec<VEC>(static_cast<const T*>(key ? a.wk : a.wq) + (a.norm == NORM_ALL ? (long)head * D : 0) + e0, g);
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) x[e] *= r * g[e];
+      for (int e = 0; e < VEC; ++e) x[e] = a.steps ? stored<T>(stored<T>(x[e] * r) * g[e]) : x[e] * (r * g[e]);
     } else {
 #pragma unroll
       for (int e = 0; e < VEC; ++e) x[e] *= r;
@@ -352,8 +364,8 @@ qkv_prep_wide_kernel(const PrepArgs a) {
         if (e0 + e < a.rot) {
           const float2 c = cs[(e0 + e) / 2];
           const float u = x[e], v = x[e + 1];
-          x[e] = u * c.x - v * c.y;
-          x[e + 1] = v * c.x + u * c.y;
+          x[e] = turn_low(u, v, c);
+          x[e + 1] = turn_high(u, v, c);
         }
       }
     } else if (a.rot) {
@@ -364,7 +376,7 @@ qkv_prep_wide_kernel(const PrepArgs a) {
         const float y = __shfl_sync(0xffffffffu, x[e], src);
         if (turn) {
           const float2 c = cs[(low ? e0 : e0 - half) + e];
-          x[e] = x[e] * c.x + (low ? -y : y) * c.y;
+          x[e] = low ? turn_low(x[e], y, c) : turn_high(y, x[e], c);
         }
       }
     }
@@ -372,7 +384,7 @@ qkv_prep_wide_kernel(const PrepArgs a) {
     if (live) {
       if (!key) {
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) x[e] *= warm;
+        for (int e = 0; e < VEC; ++e) x[e] = (a.steps ? stored<T>(stored<T>(x[e]) * a.q_mult) : x[e]) * warm;
       }
       T* dst = key ? (a.kp ? static_cast<T*>(a.kp) + (n * a.G + head / a.maps) * (TALK ? D : a.dq) : nullptr) : static_cast<T*>(a.qp) + (n * HM + head) * a.dq;
       if (TALK && !key) store_vec<VEC>(sq + head * D + e0, x);

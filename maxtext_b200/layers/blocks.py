@@ -391,7 +391,7 @@ class Attention:
                                                         and FusedParam.possible([self.q, self.k, self.v])) else None
     # everything that reads the layer input as one product [q | k | v | gate] (inference)
     self.in_parts = [p for p in (self.q, self.k, self.v, self.g) if p is not None]
-    self.qkvg = FusedParam(self.in_parts) if sizes is not None and FusedParam.possible(self.in_parts) else None
+    self.qkvg = self.qkv if sizes is None else FusedParam(self.in_parts) if FusedParam.possible(self.in_parts) else None
     self.vn = Norm(ab, "value_norm", self.dh, c.normalization_layer_epsilon, with_scale=(self.v_norm == "scale"), axes=("norm",)) if self.v_norm else None
     self.bq = self.bk = self.bv = None
     if bias:
@@ -432,7 +432,7 @@ class Attention:
     """The sink scores in the compute type, or None."""
     if isinstance(self.sinks, Constant) and self.sinks.data.dtype != dtype:
       self.sinks.data = self.sinks.data.to(dtype)
-    return self.sinks.data if self.sinks is not None else None
+    return self.sinks.data.to(dtype) if self.sinks is not None else None
 
   def _mix_scores(self, q):
     """q [B, S, H, D] -> [B, S, H, G * D]: sum_g T[h, g] (q_g . k_g) as one product with the keys of all key heads side by side."""
@@ -471,7 +471,7 @@ class Attention:
 
   def serves(self, x, ctx) -> bool:
     """Will this call run the inference kernels?"""
-    if self.sizes is None or ctx.cache is None:
+    if ctx.cache is None:
       return False
     from ..ops import cached_attention as CA
     return CA.servable(x, self, ctx)

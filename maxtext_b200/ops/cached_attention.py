@@ -1,6 +1,6 @@
 """Attention over a slot-indexed key/value cache on the inference kernels (`csrc/cached_attention_sm100.cu`).
 
-`serve` is the whole attention part of a layer with sizes of its own (`layers.blocks.HeadSizes`): one kernel adds biases, normalises, rotates,
+`serve` is the whole attention part of a layer: one kernel adds biases, normalises, rotates,
 fills the cache and lays the operands out for what follows; prompts run the flash kernel (head widths padded to the next variant), one new
 token per sequence runs the split decode kernel, and everything else (fp32, unusual widths) a plain kernel that reads the cache. Sinks,
 soft caps, windows, chunks, a query temperature, a second map per head (differential attention) and a sigmoid output gate are parameters. Where
@@ -21,13 +21,31 @@ def kernels_ok(t: torch.Tensor) -> bool:
 
 
 def servable(x, layer, ctx) -> bool:
-  """Can this call of a `layers.blocks.Attention` with sizes of its own run `serve`?"""
+  """Can this call of a `layers.blocks.Attention` run `serve`?"""
   from ..inference.kvcache import LayerKVCache
   c = ctx.cache
   return (kernels_ok(x) and type(c) is LayerKVCache and c.quant is None and c.seq_size == 1 and c.k.dtype == x.dtype and ctx.tp_size == 1
           and ctx.positions3 is None and ctx.bidir is None and layer.vn is None and (not layer.share_kv or layer.sizes is not None)
           and not (layer.qk_norm and (layer.l2_qk_norm or layer.qn.scale is None or layer.qn.offset != 0))
-          and not (ctx.segment_ids is not None and (x.dtype != torch.bfloat16 or not prompt_kernel(layer))))
+          and not (ctx.segment_ids is not None and (x.dtype != torch.bfloat16 or not prompt_kernel(layer)))
+          and (layer.sizes is not None or _plain_servable(x, layer, ctx)))
+
+
+def _plain_servable(x, layer, ctx) -> bool:
+  """The same for a layer without sizes of its own. Preparing q, k and v with separate kernels takes about 20 launches a layer (rotations with their
+  copies, two scatters into the cache, the index arithmetic of each), and a decode step 22 us (one slot), 40 us (45 slots) or 36 us (128 slots)
+  a layer longer. What `serve` does not do stays on `LayerKVCache.attend`: gated queries, fp32, rotations with fewer or more angles than rotated lanes,
+  positions or slots that are not int64, segments behind cached tokens."""
+  c, S = ctx.cache, x.shape[1]
+  rot = int(layer.rotary_dim or layer.dh)
+  longs = all(t.dtype == torch.int64 for t in (ctx.positions, c.slot_ids, c.lengths)) and (c.new_lens is None or c.new_lens.dtype == torch.int64)
+  return (x.dtype == torch.bfloat16 and not layer.gated and layer.dh <= 512 and layer.hq_l % layer.hkv_l == 0 and longs
+          and tuple(ctx.positions.shape) == tuple(x.shape[:2]) and c.slot_ids.numel() == c.lengths.numel() == x.shape[0]
+          and (c.new_lens is None or c.new_lens.numel() == x.shape[0])
+          and (not layer.use_rope or (rot % 2 == 0 and layer.inv_ts.dtype == torch.float32 and layer.inv_ts.numel() == rot // 2
+                                      and layer.inv_ts.is_contiguous()))
+          and all(n is None or n.kind == "rms" for n in (layer.qn, layer.kn))
+          and (S == 1 or ctx.segment_ids is None or ctx.mode == "prefill"))
 
 
 def flash_widths(qk: int, vd: int):
@@ -121,8 +139,12 @@ def serve(layer, q, k, v, g, ctx):
   kp = torch.empty(N, G, dq, dtype=q.dtype, device=q.device) if pack_k else None
   copy_v = pack_k and (dvp != Dv or bias[2] is not None or v.stride(0) % 8 != 0 or v.data_ptr() % 16 != 0)
   vp = torch.empty(N, G, dvp, dtype=q.dtype, device=q.device) if copy_v else None
+  # plain layers keep the roundings of their separate kernels: a prompt's keys are the same whichever path wrote them
+  steps = layer.sizes is None
   E.qkv_prep(q, k, v, D, Dv, ctx.positions.contiguous(), layer.inv_ts if rot else None, rot, eps, qp, kp, vp, cache.k, cache.v, cache.slot_ids,
-             cache.lengths, cache.new_lens, *bias, *norms, layer.interleaved, maps, *temp)
+             cache.lengths, cache.new_lens, *bias, *norms, layer.interleaved, maps, *temp, steps=steps, q_mult=scale if steps else 1.0)
+  if steps:
+    scale = 1.0
   if S == 1:
     return decode(qp, cache, scale, cap, win, sinks, g, chunk, layer)
   if apart is not None:

@@ -84,3 +84,45 @@ def test_sampling_kernel_matches_the_pytorch_definition():
     got = torch.bincount(toks, minlength=16).float() / toks.numel()
     assert (got - want).abs().max() < 0.012, (strategy, got, want)
     assert (got[want == 0] == 0).all()
+
+
+@pytest.mark.parametrize("name", ["llama3-8b", "mistral-7b", "gemma-2b", "gemma2-2b", "gemma3-4b", "qwen3-8b", "qwen2.5-7b", "gpt3-6b", "olmo3-7b",
+                                  "llama4-17b-16e", "gpt-oss-20b"])
+@pytest.mark.parametrize("head_dim", [16, 20, 128])
+def test_one_kernel_for_q_k_v_and_the_cache_matches_the_separate_ones(name, head_dim, monkeypatch):
+  """Padded prompts, single tokens and portions behind cached tokens through the layers' fused preparation and through the general path. Both
+  round to bf16 between the same products, so each is as far from the fp32 engine as the other up to the spread of single roundings."""
+  from helpers import tiny_config
+  from maxtext_b200.inference.maxengine import MaxEngine
+  from maxtext_b200.layers.blocks import Attention
+  more = [f"head_dim={head_dim}", "max_target_length=48", "max_prefill_predict_length=40", "per_device_batch_size=3", "weight_init=normal"]
+  g = torch.Generator().manual_seed(1)
+  steps = [[torch.randint(1, 256, (n,), generator=g).tolist() for n in ns] for ns in ((9, 14, 3), (1, 1, 1), (1, 1, 1), (5, 2, 7), (1, 1, 1))]
+  weights = None
+
+  def logits(dtype, served):
+    nonlocal weights
+    used = []
+    real = Attention.serves
+    monkeypatch.setattr(Attention, "serves", lambda self, x, ctx: used.append(served and real(self, x, ctx)) or used[-1])
+    eng = MaxEngine(tiny_config(name, extra=more + [f"dtype={dtype}", "hardware=gpu"]), device="cuda")
+    eng.load_params(seed=3)
+    if weights is None:
+      weights = eng.model.store.master.clone()
+    eng.model.store.master.copy_(weights)
+    eng.model.store.sync_compute_from_master()
+    state = eng.init_decode_state(3)
+    out = [eng.extend(state, [0, 1, 2], toks).float() for toks in steps]
+    monkeypatch.setattr(Attention, "serves", real)
+    return torch.stack(out), any(used), state.caches
+
+  want, _, _ = logits("float32", False)
+  general, _, kept = logits("bfloat16", False)
+  fused, ran, kept2 = logits("bfloat16", True)
+  assert ran
+  err = lambda a: float((a - want).norm() / want.norm())  # noqa: E731
+  assert err(fused) <= 1.5 * err(general) + 2 ** -8, (err(fused), err(general))
+  for a, b in zip(kept, kept2):
+    for n in ("k", "v"):
+      x, y = getattr(a[0], n).float(), getattr(b[0], n).float()
+      assert torch.equal(x == 0, y == 0) and float((x - y).norm() / x.norm()) <= 2 ** -5
