@@ -9,8 +9,9 @@
 extern "C" {
 int mt_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_mn, int b_mn,
                  int out_f32, int accumulate, int* status, int num_sms, cudaStream_t stream);
-int mt_rmsnorm_fwd(const void* x, const void* scale, float eps, float offset, void* y, float* rstd, int rows, int D, cudaStream_t st);
-int mt_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const float* rstd, float offset, void* dx, float* dscale,
+int mt_rmsnorm_fwd(const void* x, const void* add, void* sum, const void* scale, float eps, float offset, void* y, float* rstd, int rows, int D,
+                   cudaStream_t st);
+int mt_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const float* rstd, float offset, const void* dres, void* dx, float* dscale,
                    float* partial, int rows, int D, int sms, cudaStream_t st);
 int mt_rmsnorm_bwd_partial_rows(int rows, int D, int sms);
 int mt_rope(void* x, const int* pos, const float* inv_ts, long tokens, int heads, int dh, int n_rot, int rot_dim, int interleaved,
@@ -203,23 +204,25 @@ int64_t kernel_status(bool reset) {
 }
 
 void rmsnorm_fwd(const torch::Tensor& x, const c10::optional<torch::Tensor>& scale, double eps, double offset, torch::Tensor& y,
-                 const c10::optional<torch::Tensor>& rstd) {
-  TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && x.dim() == 2);
+                 const c10::optional<torch::Tensor>& rstd, const c10::optional<torch::Tensor>& add, const c10::optional<torch::Tensor>& sum) {
+  TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && x.dim() == 2 && bool(add) == bool(sum));
+  for (const auto& t : {add, sum}) TORCH_CHECK(!t || (t->is_contiguous() && t->numel() == x.numel() && t->scalar_type() == x.scalar_type()));
   c10::cuda::CUDAGuard guard(x.device());
-  check(mt_rmsnorm_fwd(x.data_ptr(), scale ? scale->data_ptr() : nullptr, (float)eps, (float)offset, y.data_ptr(),
+  check(mt_rmsnorm_fwd(x.data_ptr(), add ? add->data_ptr() : nullptr, sum ? sum->data_ptr() : nullptr, scale ? scale->data_ptr() : nullptr, (float)eps, (float)offset, y.data_ptr(),
                        rstd ? rstd->data_ptr<float>() : nullptr, (int)x.size(0), (int)x.size(1), cur_stream()),
         "mt_rmsnorm_fwd");
 }
 
 void rmsnorm_bwd(const torch::Tensor& dy, const torch::Tensor& x, const c10::optional<torch::Tensor>& scale, const torch::Tensor& rstd,
-                 double offset, torch::Tensor& dx, const c10::optional<torch::Tensor>& dscale) {
+                 double offset, torch::Tensor& dx, const c10::optional<torch::Tensor>& dscale, const c10::optional<torch::Tensor>& dres) {
   TORCH_CHECK(x.is_contiguous() && dy.is_contiguous() && dx.is_contiguous());
+  TORCH_CHECK(!dres || (dres->is_contiguous() && dres->numel() == x.numel() && dres->scalar_type() == x.scalar_type()));
   c10::cuda::CUDAGuard guard(x.device());
   torch::Tensor partial;
   if (dscale) partial = torch::empty({mt_rmsnorm_bwd_partial_rows((int)x.size(0), (int)x.size(1), num_sms()), x.size(1)},
                                      torch::TensorOptions().dtype(torch::kFloat32).device(x.device()));
   check(mt_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), scale ? scale->data_ptr() : nullptr, rstd.data_ptr<float>(), (float)offset,
-                       dx.data_ptr(), dscale ? dscale->data_ptr<float>() : nullptr, dscale ? partial.data_ptr<float>() : nullptr,
+                       dres ? dres->data_ptr() : nullptr, dx.data_ptr(), dscale ? dscale->data_ptr<float>() : nullptr, dscale ? partial.data_ptr<float>() : nullptr,
                        (int)x.size(0), (int)x.size(1), num_sms(), cur_stream()),
         "mt_rmsnorm_bwd");
 }
@@ -319,8 +322,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_set_group_m", [](int64_t v) { TORCH_CHECK(mt_gemm_set_group_m((int)v) == 0, "bad group size"); });
   m.def("kernel_status", &kernel_status);
   m.def("launch_count", &launch_count);
-  m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("rmsnorm_fwd", &rmsnorm_fwd, py::arg("x"), py::arg("scale"), py::arg("eps"), py::arg("offset"), py::arg("y"), py::arg("rstd"),
+        py::arg("add") = py::none(), py::arg("sum") = py::none());
+  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("dy"), py::arg("x"), py::arg("scale"), py::arg("rstd"), py::arg("offset"), py::arg("dx"), py::arg("dscale"),
+        py::arg("dres") = py::none());
   m.def("rope_inplace", &rope_inplace);
   m.def("gated_act_fwd", &gated_act_fwd);
   m.def("gated_act_bwd", &gated_act_bwd);

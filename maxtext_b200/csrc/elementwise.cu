@@ -46,10 +46,13 @@ __device__ __forceinline__ float row_sum(float v, float* smem) {
 }
 
 // ------------------------------------------------------------------------------------------------ RMSNorm forward
-// y = bf16(x * rstd) * bf16(scale + offset), both roundings as in the reference layer.
-template <int TPR, int VPT>
-__global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ scale, float eps,
-                                   float offset, __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int rows, int D) {
+// y = bf16(x * rstd) * bf16(scale + offset), both roundings as in the reference layer. With `add` the row is bf16(x + add), which also goes to
+// `sum`: the residual add in front of a norm, in the norm's own pass. Bandwidth-bound; at 16384 rows of 4096 lanes the add and the norm took 65 + 85 us
+// as two kernels (402 + 268 MB) and take 117 us as one (537 MB).
+template <int TPR, int VPT, bool ADD>
+__global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ add, __nv_bfloat16* __restrict__ sum,
+                                   const __nv_bfloat16* __restrict__ scale, float eps, float offset, __nv_bfloat16* __restrict__ y,
+                                   float* __restrict__ rstd_out, int rows, int D) {
   __shared__ float red[8];
   const int rows_per_block = blockDim.x / TPR;
   const int r_in_block = threadIdx.x / TPR;
@@ -62,8 +65,16 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
   for (int i = 0; i < VPT; ++i) {
     const int col = (i * TPR + tid) * 8;
     if (active && col < D) {
-      bf16x8 p = *reinterpret_cast<const bf16x8*>(x + row * D + col);
-      unpack8(p, v[i]);
+      unpack8(*reinterpret_cast<const bf16x8*>(x + row * D + col), v[i]);
+      if (ADD) {
+        float a[8];
+        unpack8(*reinterpret_cast<const bf16x8*>(add + row * D + col), a);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[i][e] += a[e];
+        const bf16x8 p = pack8(v[i]);
+        *reinterpret_cast<bf16x8*>(sum + row * D + col) = p;
+        unpack8(p, v[i]);                                  // the norm reads the stream as it is stored
+      }
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss += v[i][e] * v[i][e];
     }
@@ -91,14 +102,16 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
 }
 
 // ------------------------------------------------------------------------------------------------ RMSNorm backward
-// dx = rstd * (g - xhat * mean(g * xhat)), g = dy * (scale + offset);  dscale += sum_rows dy * xhat.
+// dx = rstd * (g - xhat * mean(g * xhat)) [+ dres], g = dy * (scale + offset);  dscale += sum_rows dy * xhat. `dres` is what reaches the same row past
+// the norm (the residual stream's own gradient): added here, in fp32, it costs no pass of its own.
 // Blocks stride over rows and keep per-column dscale partials in registers; the warps of a block that work on rows of their own
 // (TPR 32) add theirs up in shared memory, each block writes one row into `partial`, and rms_dscale_reduce_kernel adds the rows up
 // in a fixed order: no atomics, so the result is bitwise reproducible.
 template <int TPR, int VPT>
 __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                    const __nv_bfloat16* __restrict__ scale, const float* __restrict__ rstd_in, float offset,
-                                   __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int D) {
+                                   const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows,
+                                   int D) {
   __shared__ float red[8];
   const int rows_per_block = blockDim.x / TPR;
   const int r_in_block = threadIdx.x / TPR;
@@ -151,6 +164,12 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const _
         float o[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] = rstd * (g[i][e] - xh[i][e] * dot);
+        if (dres) {
+          float a[8];
+          unpack8(*reinterpret_cast<const bf16x8*>(dres + row * D + col), a);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] += a[e];
+        }
         *reinterpret_cast<bf16x8*>(dx + row * D + col) = pack8(o);
       }
     }
@@ -225,8 +244,9 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict
     for (int h = 0; h < n_rot; ++h) {
       const float a = __bfloat162float(base[h * dh + i0]);
       const float b = __bfloat162float(base[h * dh + i1]);
-      base[h * dh + i0] = __float2bfloat16_rn(a * c - b * s);
-      base[h * dh + i1] = __float2bfloat16_rn(b * c + a * s);
+      // written out like the rotation of the inference kernels, so that both round alike
+      base[h * dh + i0] = __float2bfloat16_rn(__fmaf_rn(a, c, -__fmul_rn(b, s)));
+      base[h * dh + i1] = __float2bfloat16_rn(__fmaf_rn(a, s, __fmul_rn(b, c)));
     }
   }
 }
@@ -316,23 +336,26 @@ __global__ void embedding_bwd_kernel(const int* __restrict__ tok, const __nv_bfl
 using namespace mt;
 
 template <int TPR>
-static void launch_rms_fwd(const void* x, const void* scale, float eps, float offset, void* y, float* rstd, int rows, int D,
+static void launch_rms_fwd(const void* x, const void* add, void* sum, const void* scale, float eps, float offset, void* y, float* rstd, int rows, int D,
                            cudaStream_t st) {
   const int vpt = (D / 8 + TPR - 1) / TPR;
   const int threads = 256;
   const int rpb = threads / TPR;
   const int grid = (rows + rpb - 1) / rpb;
-#define L(V) rmsnorm_fwd_kernel<TPR, V><<<grid, threads, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)scale, eps, offset, \
-                                                                  (__nv_bfloat16*)y, rstd, rows, D)
+#define K(V, A) rmsnorm_fwd_kernel<TPR, V, A><<<grid, threads, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)add, (__nv_bfloat16*)sum, \
+                                                                        (const __nv_bfloat16*)scale, eps, offset, (__nv_bfloat16*)y, rstd, rows, D)
+#define L(V) do { if (add) K(V, true); else K(V, false); } while (0)
   if (vpt <= 1) L(1); else if (vpt <= 2) L(2); else if (vpt <= 4) L(4); else L(8);
 #undef L
+#undef K
 }
 
-extern "C" int mt_rmsnorm_fwd(const void* x, const void* scale, float eps, float offset, void* y, float* rstd, int rows, int D,
-                              cudaStream_t st) {
-  if (D % 8 || D > 8 * 256 * 8) return -1;
-  if (D <= 512) launch_rms_fwd<32>(x, scale, eps, offset, y, rstd, rows, D, st);
-  else launch_rms_fwd<256>(x, scale, eps, offset, y, rstd, rows, D, st);
+// add, sum: both null, or the residual add in front of the norm
+extern "C" int mt_rmsnorm_fwd(const void* x, const void* add, void* sum, const void* scale, float eps, float offset, void* y, float* rstd, int rows,
+                              int D, cudaStream_t st) {
+  if (D % 8 || D > 8 * 256 * 8 || !add != !sum) return -1;
+  if (D <= 512) launch_rms_fwd<32>(x, add, sum, scale, eps, offset, y, rstd, rows, D, st);
+  else launch_rms_fwd<256>(x, add, sum, scale, eps, offset, y, rstd, rows, D, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -344,15 +367,15 @@ static int rms_bwd_grid(int rows, int tpr, int sms) {
 }
 
 template <int TPR>
-static void launch_rms_bwd(const void* dy, const void* x, const void* scale, const float* rstd, float offset, void* dx, float* dscale,
-                           float* partial, int rows, int D, int sms, cudaStream_t st) {
+static void launch_rms_bwd(const void* dy, const void* x, const void* scale, const float* rstd, float offset, const void* dres, void* dx,
+                           float* dscale, float* partial, int rows, int D, int sms, cudaStream_t st) {
   const int vpt = (D / 8 + TPR - 1) / TPR;
   const int threads = 256;
   const int grid = rms_bwd_grid(rows, TPR, sms);
   float* part = dscale ? partial : nullptr;
 #define L(V) rmsnorm_bwd_kernel<TPR, V><<<grid, threads, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,                 \
-                                                                  (const __nv_bfloat16*)scale, rstd, offset, (__nv_bfloat16*)dx,    \
-                                                                  part, rows, D)
+                                                                  (const __nv_bfloat16*)scale, rstd, offset,                        \
+                                                                  (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, part, rows, D)
   if (vpt <= 1) L(1); else if (vpt <= 2) L(2); else if (vpt <= 4) L(4); else L(8);
 #undef L
   if (part) rms_dscale_reduce_kernel<<<(D + 31) / 32, 32 * kDsLanes, 0, st>>>(part, grid, D, dscale);
@@ -366,11 +389,11 @@ extern "C" int mt_rmsnorm_bwd_partial_rows(int rows, int D, int sms) {
 
 // `partial`: scratch of mt_rmsnorm_bwd_partial_rows(rows, D, sms) x D floats (needed only when dscale is given); every block writes
 // its row, so the scratch needs no clearing.
-extern "C" int mt_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const float* rstd, float offset, void* dx,
-                              float* dscale, float* partial, int rows, int D, int sms, cudaStream_t st) {
+extern "C" int mt_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const float* rstd, float offset, const void* dres,
+                              void* dx, float* dscale, float* partial, int rows, int D, int sms, cudaStream_t st) {
   if (D % 8 || D > 8 * 256 * 8 || (dscale && !partial)) return -1;
-  if (D <= 512) launch_rms_bwd<32>(dy, x, scale, rstd, offset, dx, dscale, partial, rows, D, sms, st);
-  else launch_rms_bwd<256>(dy, x, scale, rstd, offset, dx, dscale, partial, rows, D, sms, st);
+  if (D <= 512) launch_rms_bwd<32>(dy, x, scale, rstd, offset, dres, dx, dscale, partial, rows, D, sms, st);
+  else launch_rms_bwd<256>(dy, x, scale, rstd, offset, dres, dx, dscale, partial, rows, D, sms, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -73,7 +73,7 @@ class LayerCtx:
   positions3: torch.Tensor | None = None  # [B, S, 3] (temporal, height, width) positions of a multimodal prompt (`use_mrope`)
   deepstack: tuple | None = None     # (image mask [B, S], [features [B, N*K, D], ...]): feature i is added after decoder layer i
   new_lens: torch.Tensor | None = None  # [B] real tokens per row of a right-padded inference batch (None: all of them)
-  next_norm: object = None           # fp32 residual streams: the norm that reads the stream after the current layer ...
+  next_norm: object = None           # inference: the norm that reads the stream after the current layer ...
   normed: torch.Tensor | None = None  # ... and its output, handed from the layer that computed it to the one that reads it
   origin: torch.Tensor | None = None  # models whose layers run in a loop: the embedding output in the compute type, which every pass reads again ...
   beside: torch.Tensor | None = None  # ... and (inference) the rows [stream | embedding output] that it reads them from

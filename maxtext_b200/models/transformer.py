@@ -225,18 +225,37 @@ class DecoderBlock:
       return self._call_gated_stream(x, ctx)
     if self.plan.residual_fp32:
       return self._call_fp32_stream(x, ctx) if self.n1b is not None else self._call_joined_stream(x, ctx)
-    a = self.attn(self.n1(x) if self.n1 is not None else x, ctx)
+    if ctx.normed is not None:                # the layer before has normalised the stream already
+      h, ctx.normed = ctx.normed, None
+    elif self.n1 is not None:
+      x, h = F.add_norm(x, None, self.n1)
+    else:
+      h = x
+    a = self.attn(h, ctx)
     if self.n1b is not None:
       a = self.n1b(a)
-    x = x + ctx.dropout(a, 0)                 # src/maxtext/models/llama2.py: dropout on each residual branch
-    h = self.n2(x) if self.n2 is not None else x
+    a = ctx.dropout(a, 0)                     # src/maxtext/models/llama2.py: dropout on each residual branch
+    if self.n2 is not None:
+      x, h = F.add_norm(x, a, self.n2)
+    else:
+      x = h = x + a
     m = self.mlp(h, ctx, original=x) if self.plan.mlp == "gemma4_moe" else self.mlp(h, ctx)
     if self.n2b is not None:
       m = self.n2b(m)
-    x = x + ctx.dropout(m, 1)
+    m = ctx.dropout(m, 1)
+    if ctx.next_norm is not None:
+      x, ctx.normed = F.add_norm(x, m, ctx.next_norm)
+      return x
+    x = x + m
     if self.layer_scalar is not None:
       x = x * self.layer_scalar.leaf().to(x.dtype)
     return x
+
+  def plain_stream(self) -> bool:
+    """Does this block read and write one residual stream in the compute type, with nothing in front of its norm or behind its last add? (Then the
+    norm that reads the stream next can join that add.)"""
+    return (self.engram is None and self.mhc_attn is None and self.hc1 is None and not self.plan.residual_gate and not self.plan.residual_fp32
+            and self.layer_scalar is None)
 
   def reader(self):
     """What reads the residual stream first in this block: its norm, with the weights of the streams where there are several."""
@@ -689,6 +708,16 @@ class Transformer:
     h = normed if normed is not None else self.final_norm(x)
     return F.head_logits(h, self.head_param(), self.config.final_logits_soft_cap, self.head_logit_scale(), fp32_out=self.family.residual_fp32)
 
+  def _next_plain_norm(self, i: int, ctx: LayerCtx, logit_rows):
+    """The norm that joins the last residual add of running layer i (inference, plain streams), or None. After the last layer only where every row
+    goes on to the head."""
+    plain = lambda layer: len(layer.blocks) == 1 and layer.entry is None and layer.blocks[0].plain_stream()  # noqa: E731
+    if ctx.deepstack is not None or ctx.batch_split > 1 or not plain(self.runs[i]):
+      return None
+    if i + 1 < len(self.runs):
+      return self.runs[i + 1].blocks[0].n1 if plain(self.runs[i + 1]) else None
+    return self.final_norm if logit_rows is None and isinstance(self.final_norm, L.Norm) else None
+
   # ------------------------------------------------------------------ plain forward (eval / inference / tests)
   @torch.no_grad()
   def forward(self, tokens, positions=None, segment_ids=None, mode="train", caches=None, images=None, image_mask=None, positions3=None,
@@ -727,6 +756,8 @@ class Transformer:
       ctx.cache = caches[i] if caches is not None else None
       if self.family.residual_fp32 and not torch.is_grad_enabled():
         ctx.next_norm = self.runs[i + 1].reader(ctx) if i + 1 < len(self.runs) else self.final_norm.reader()
+      elif not torch.is_grad_enabled():
+        ctx.next_norm = self._next_plain_norm(i, ctx, logit_rows)
       x = layer(x, ctx)
     normed = ctx.normed
     if logit_rows is None:

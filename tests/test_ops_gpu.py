@@ -47,6 +47,48 @@ def test_rmsnorm_scale_gradient_adds_every_row_once(rows, D):
   assert bool(((ds.double() - 3.0 - terms.sum(0)).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("rows,D,offset", [(1, 8, 0.0), (5, 512, 1.0), (3, 520, 0.0), (300, 2048, 0.0), (17, 16384, 1.0)])
+def test_residual_add_and_norm_in_one_pass(rows, D, offset):
+  """The pair (x + a, norm of it) is the same bits as the add and the norm on their own; its gradient is the stream's plus the norm's, rounded once:
+  within one bf16 ulp (2**-8) of the sum of the two, which the separate kernels round three times."""
+  from maxtext_b200.layers.blocks import Constant
+  from maxtext_b200.ops import functional as F
+  g = torch.Generator(device="cuda").manual_seed(rows)
+  x, a, dx, dy = (torch.randn(rows, D, device="cuda", generator=g).bfloat16() for _ in range(4))
+
+  class Scale(Constant):
+    shape, main_grad, grad_written = (D,), None, False
+
+  class Norm:
+    kind, eps, scale = "rms", 1e-5, Scale((1 + 0.1 * torch.randn(D, device="cuda", generator=g)).bfloat16())
+  Norm.offset = offset
+
+  def plain(s):
+    y, rstd = torch.empty_like(s), torch.empty(rows, device="cuda")
+    _E().rmsnorm_fwd(s, Norm.scale.data, 1e-5, offset, y, rstd)
+    return y, rstd
+  for add in (a, None):
+    want = x if add is None else x + a
+    y, rstd = plain(want)
+    with torch.no_grad():
+      s, h = F.add_norm(x, add, Norm)
+    assert torch.equal(s, want) and torch.equal(h, y)
+    xr, ar = x.clone().requires_grad_(True), a.clone().requires_grad_(True)
+    s, h = F.add_norm(xr, None if add is None else ar, Norm)
+    assert torch.equal(s, want) and torch.equal(h, y)
+    torch.autograd.backward([s, h], [dx, dy])
+    through = torch.empty_like(x)
+    _E().rmsnorm_bwd(dy, want, Norm.scale.data, rstd, offset, through, None)
+    exact = through.float() + dx.float()
+    assert bool(((xr.grad.float() - exact).abs() <= 2 ** -8 * (exact.abs() + through.float().abs()) + 1e-6).all())
+    if add is not None:
+      assert torch.equal(ar.grad, xr.grad)
+    s, h = F.add_norm(xr, None if add is None else ar, Norm)       # only the stream, or only the norm, is used
+    assert torch.equal(torch.autograd.grad(s, xr, dx)[0], dx)
+    s, h = F.add_norm(xr, None if add is None else ar, Norm)
+    assert torch.equal(torch.autograd.grad(h, xr, dy)[0], through)
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 def test_rope_roundtrip_and_reference(interleaved):
   E = _E()
