@@ -86,7 +86,8 @@ bool gemm_supported(const torch::Tensor& a, const torch::Tensor& b, const torch:
   const int64_t M = ta ? a.size(1) : a.size(0), K = ta ? a.size(0) : a.size(1), N = tb ? b.size(0) : b.size(1);
   if ((tb ? b.size(1) : b.size(0)) != K || out.size(0) != M || out.size(1) != N) return false;
   // M is a contiguous dimension only of a transposed A; elsewhere TMA clips the ragged last row block
-  return M >= 128 && N >= 128 && K >= 64 && (!ta || M % 8 == 0) && N % 8 == 0 && K % 8 == 0;
+  // (K is contiguous in an operand unless both are transposed: a weight gradient sums over any number of tokens, the last ones of a step clipped likewise)
+  return M >= 128 && N >= 128 && K >= 64 && (!ta || M % 8 == 0) && N % 8 == 0 && ((ta && !tb) || K % 8 == 0);
 }
 
 extern "C" int mt_gemm_small_m_supported(int M, int N, int K, long ldx, long ldw, long ldo);

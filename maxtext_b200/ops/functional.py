@@ -48,8 +48,9 @@ def _small_m_wins(M, N, K) -> bool:
   return M <= 32 and N <= 4096 and K <= 4096
 
 
-def _gemm_supported(M, N, K, a, b):
-  return a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and K % 8 == 0 and N % 8 == 0 and K >= 16
+def _gemm_supported(M, N, K, a, b, k_strided=False):
+  """`k_strided`: the summed dimension is the slow one of both operands (a weight gradient), so that its length needs no alignment."""
+  return a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and (k_strided or K % 8 == 0) and N % 8 == 0 and K >= 16
 
 
 def mm(a: torch.Tensor, b: torch.Tensor, ta: bool, tb: bool, out: torch.Tensor | None = None,
@@ -71,7 +72,7 @@ def mm(a: torch.Tensor, b: torch.Tensor, ta: bool, tb: bool, out: torch.Tensor |
         and E.gemm_small_m_supported(a, b, out)):
       E.gemm_small_m(a, b, out)            # decode-sized products stream the weight once (csrc/gemm_small_m.cu)
       return out
-    if _GEMM_IMPL == "tcgen05" and _gemm_supported(M, N, K, a, b) and E.gemm_supported(a, b, out, ta, tb):
+    if _GEMM_IMPL == "tcgen05" and _gemm_supported(M, N, K, a, b, ta and not tb) and E.gemm_supported(a, b, out, ta, tb):
       E.gemm(a, b, out, ta, tb, accumulate)
       return out
     if _GEMM_IMPL == "tcgen05":

@@ -139,3 +139,11 @@ def test_small_m_gemm_strided_views_and_dispatch():
   assert (y.float() - ref2).abs().max().item() <= 2e-2 * ref2.abs().max().item()
   # K not a multiple of 64 is not covered: the caller falls back and counts it
   assert not E.gemm_small_m_supported(xb[:, :40].contiguous(), wb[:, :40].contiguous(), torch.empty(12, 300, device="cuda", dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("K", [65, 71, 1999, 5997])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_gemm_weight_gradient_over_any_number_of_rows(K, accumulate):
+  """The summed dimension of a weight gradient is the slow one of both operands: its last step is clipped, whatever its length."""
+  _run(136, 264, K, True, False, torch.float32, accumulate)                # 128-row tiles
+  _run(768, 512, K, True, False, torch.float32, accumulate)                # CTA pairs
