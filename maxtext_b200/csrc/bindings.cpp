@@ -28,6 +28,9 @@ int mt_amax(const void* x, long n, float* amax, int sms, cudaStream_t st);
 int mt_quantize_fp8(const void* x, int R, int C, const float* amax, int fmt, void* q, void* qt, float* dequant, cudaStream_t st);
 int mt_gemm_fp8(const void* a, const void* b, void* c, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_fmt, int b_fmt,
                 int out_f32, int accumulate, const float* scale_a, const float* scale_b, int* status, int num_sms, cudaStream_t stream);
+int mt_gemm_narrow_width(int M, int N, int num_sms);
+int mt_gemm_narrow(const void* a, const void* b, void* c, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int* status, int num_sms,
+                   cudaStream_t stream);
 int mt_gemm_set_group_m(int v);
 int mt_gemm_set_raster(int v);
 int mt_gemm_bf16_pair(const void* a, const void* b, void* c, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_mn, int b_mn,
@@ -119,6 +122,12 @@ void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bo
   const int64_t M = ta ? a.size(1) : a.size(0), K = ta ? a.size(0) : a.size(1), N = tb ? b.size(0) : b.size(1);
   const bool f32 = out.scalar_type() == torch::kFloat32;
   TORCH_CHECK(!accumulate || f32, "gemm: accumulate requires an fp32 output");
+  if (!ta && tb && !f32 && mt_gemm_narrow_width((int)M, (int)N, num_sms()) > 0) {
+    check(mt_gemm_narrow(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0), out.stride(0),
+                         status_tensor().data_ptr<int>(), num_sms(), cur_stream()),
+          "mt_gemm_narrow");
+    return;
+  }
   if (g_use_pair && N % 256 == 0 && M >= 512) {
     int rc = mt_gemm_bf16_pair(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0), out.stride(0),
                                ta ? 1 : 0, tb ? 0 : 1, f32 ? 1 : 0, accumulate ? 1 : 0, status_tensor().data_ptr<int>(), num_sms(),

@@ -1015,6 +1015,127 @@ static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
+// ------------------------------------------------------------------------------------------------ few rows, or few tiles
+// y = x W^T (bf16) where the tiles of the kernels above leave most of the machine idle: decoding with 128 to a few hundred slots, short prompts. One
+// 128 x BN tile per CTA, with BN (a multiple of 16) chosen so that one wave of CTAs covers the output; the ring holds as many stages as fit. Each element
+// is summed over K in one accumulator, 16 at a time, as above: the results are the same bits. What bounds it is the chain of one step of 64 after the other
+// (two waits, two copies, four MMAs, a commit) until the weights' trip from HBM takes longer. The threads that issue are picked with elect.sync: behind
+// `lane == 0` the compiler does not know that they run alone, and a step took 518 cycles whatever its bytes (371 without its MMAs): 15.5 us for
+// the average of a decode step's four products at 128 rows (K 2048 / N 4096, 2048, 11008; K 5504 / N 2048), 10.3 us now, against 23.1 us with 256-wide
+// tiles on 8 - 43 CTAs.
+struct NarrowParams {
+  int M, N, K, bn, stages, m_blocks, tmem_cols;
+  __nv_bfloat16* c;
+  long ldc;
+  int* status;
+};
+
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const NarrowParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+  // [barriers, 1 KB][A stages][B stages]
+  auto full_bar = [&](int s) { return base + 8u * s; };
+  auto empty_bar = [&](int s) { return base + 8u * (16 + s); };
+  const uint32_t done_bar = base + 256, tmem_slot = base + 264;
+  volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gen + 264);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 272);
+  volatile int* epi_ok = abort_flag + 1;
+  const uint32_t a_bytes = BM * 128, b_bytes = (uint32_t)p.bn * 128;
+  const uint32_t a0 = base + 1024, b0 = a0 + p.stages * a_bytes;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = (int)(blockIdx.x % p.m_blocks) * BM, n0 = (int)(blockIdx.x / p.m_blocks) * p.bn;
+  const int num_kb = (p.K + BK - 1) / BK;
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(done_bar, 1);
+    fence_barrier_init();
+    prefetch_tensormap(&map_a);
+    prefetch_tensormap(&map_b);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, p.tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_ptr;
+  if (warp == 0) {
+    if (elect_one()) {
+      int s = 0;
+      uint32_t phase = 0;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait(empty_bar(s), phase ^ 1, abort_flag, p.status, ST_TIMEOUT_PRODUCER)) break;
+        mbar_arrive_expect_tx(full_bar(s), a_bytes + b_bytes);
+        tma_load_2d(b0 + s * b_bytes, &map_b, full_bar(s), kb * BK, n0);
+        tma_load_2d(a0 + s * a_bytes, &map_a, full_bar(s), kb * BK, m0);
+        if (++s == p.stages) { s = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(BM, (uint32_t)p.bn, false, false);
+      int s = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait(full_bar(s), phase, abort_flag, p.status, ST_TIMEOUT_MMA)) { ok = false; break; }
+        tc_fence_after();
+        const uint64_t da = make_smem_desc(a0 + s * a_bytes, 16, 1024), db = make_smem_desc(b0 + s * b_bytes, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_ss(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+        umma_commit(empty_bar(s));
+        if (++s == p.stages) { s = 0; phase ^= 1; }
+      }
+      if (ok) umma_commit(done_bar);
+    }
+  } else {
+    const int q = warp & 3, et = threadIdx.x - 64;
+    if (et == 0) *epi_ok = mbar_wait(done_bar, 0, abort_flag, p.status, ST_TIMEOUT_EPILOGUE) ? 1 : 0;
+    named_bar_sync(3, EPI_THREADS);
+    if (*epi_ok) {
+      tc_fence_after();
+      const int row = m0 + q * 32 + lane;
+      if (m0 + q * 32 < p.M) {                 // a warp whose rows all lie below the matrix has nothing to read
+        __nv_bfloat16* out = p.c + (long)row * p.ldc;
+        for (int c = 0; c < p.bn; c += 16) {
+          uint32_t r[16];
+          tmem_ld_32x32b_x16(tmem + c + ((uint32_t)(q * 32) << 16), r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (row < p.M && n0 + c + 8 * h < p.N) {          // N is a multiple of 8
+              uint4 v;
+              v.x = pack_bf16(__uint_as_float(r[8 * h]), __uint_as_float(r[8 * h + 1]));
+              v.y = pack_bf16(__uint_as_float(r[8 * h + 2]), __uint_as_float(r[8 * h + 3]));
+              v.z = pack_bf16(__uint_as_float(r[8 * h + 4]), __uint_as_float(r[8 * h + 5]));
+              v.w = pack_bf16(__uint_as_float(r[8 * h + 6]), __uint_as_float(r[8 * h + 7]));
+              *reinterpret_cast<uint4*>(out + n0 + c + 8 * h) = v;
+            }
+          }
+        }
+      }
+    }
+  }
+  if (*abort_flag) {
+    // a wait ran out: give copies in flight time to land before shared memory is released
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) { }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, p.tmem_cols);
+  }
+}
+
 }  // namespace mt
 
 // Same contract as mt_gemm_bf16, computed by CTA pairs (cta_group::2). N must be a multiple of 128 so that every CTA's half
@@ -1067,4 +1188,43 @@ extern "C" int mt_gemm_fp8_pair(const void* a, const void* b, void* c, int M, in
   p.raster_n = pick_raster(M, N);
   return out_f32 ? launch_pair<false, false, float, true>(ma, mb, mc, p, num_sms, stream)
                  : launch_pair<false, false, __nv_bfloat16, true>(ma, mb, mc, p, num_sms, stream);
+}
+
+// The tile width with which one wave of 128 x bn tiles covers [M, N], or 0: no such width, or the kernels above take in no more per SM than this one
+// would. Their cost in the same unit (rows of operands that an SM takes in, per element of K): 256 for each wave of CTA pairs over 256 x 256 tiles, 384
+// (256) for each wave of 128 x 256 (128 x 128) tiles. Below 128 rows the library's kernels are ahead (11 against 17 us at K 2048 / N 4096).
+extern "C" int mt_gemm_narrow_width(int M, int N, int num_sms) {
+  const int m_blocks = (M + mt::BM - 1) / mt::BM;
+  if (M < 128 || N < 128 || m_blocks > num_sms) return 0;
+  const int cols = num_sms / m_blocks;                         // CTAs along N
+  const int bn = ((N + cols - 1) / cols + 15) / 16 * 16;
+  if (bn > 256) return 0;
+  const int w = N % 256 == 0 || N > 1024 ? 256 : 128;
+  const long pair_tiles = (long)((M + 255) / 256) * ((N + 255) / 256), tiles = (long)m_blocks * ((N + w - 1) / w);
+  const long present = M >= 512 && N % 256 == 0 ? (pair_tiles + num_sms / 2 - 1) / (num_sms / 2) * 256 : (tiles + num_sms - 1) / num_sms * (128 + w);
+  return (128 + bn) * 10 <= present * 9 ? bn : 0;
+}
+
+// c[M, N] = a[M, K] b[N, K]^T, bf16, for shapes with mt_gemm_narrow_width(M, N) > 0. Leading strides are multiples of 8, N and K too.
+extern "C" int mt_gemm_narrow(const void* a, const void* b, void* c, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int* status, int num_sms,
+                              cudaStream_t stream) {
+  using namespace mt;
+  const int bn = mt_gemm_narrow_width(M, N, num_sms);
+  if (bn == 0 || N % 8 || K % 8 || K < 16 || lda % 8 || ldb % 8 || ldc % 8) return -10;
+  NarrowParams p{};
+  p.M = M; p.N = N; p.K = K; p.bn = bn; p.c = static_cast<__nv_bfloat16*>(c); p.ldc = ldc; p.status = status;
+  p.m_blocks = (M + BM - 1) / BM;
+  p.tmem_cols = bn <= 32 ? 32 : bn <= 64 ? 64 : bn <= 128 ? 128 : 256;
+  constexpr int ROOM = 218 * 1024, HEAD = 2 * 1024;            // stages; barriers and alignment. 220 of 227 KB
+  const int stage = (BM + bn) * 128, num_kb = (K + BK - 1) / BK;
+  p.stages = ROOM / stage;
+  if (p.stages > 16) p.stages = 16;
+  if (p.stages > num_kb) p.stages = num_kb;
+  CUtensorMap ma, mb;
+  int e = make_map_2d(&ma, a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, lda, BK, BM);
+  if (e) return 100 + e;
+  if ((e = make_map_2d(&mb, b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldb, BK, bn))) return 200 + e;
+  if (cudaFuncSetAttribute(gemm_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROOM + HEAD) != cudaSuccess) return -2;
+  gemm_narrow_kernel<<<p.m_blocks * ((N + bn - 1) / bn), NUM_THREADS, HEAD + p.stages * stage, stream>>>(ma, mb, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -147,3 +147,17 @@ def test_gemm_weight_gradient_over_any_number_of_rows(K, accumulate):
   """The summed dimension of a weight gradient is the slow one of both operands: its last step is clipped, whatever its length."""
   _run(136, 264, K, True, False, torch.float32, accumulate)                # 128-row tiles
   _run(768, 512, K, True, False, torch.float32, accumulate)                # CTA pairs
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 2048, 2048), (129, 2056, 72), (333, 4096, 1032), (200, 136, 64), (1000, 576, 2048), (4096, 576, 128), (640, 1024, 520)])
+def test_gemm_one_wave_of_narrow_tiles(M, N, K):
+  """Shapes that leave most SMs without a wide tile: ragged rows, widths and depths, and the same bits as the CTA-pair kernel, which sums in the same
+  order."""
+  _run(M, N, K, False, True, torch.bfloat16)
+  if M >= 256 and N % 128 == 0:
+    E = _ext()
+    a, b = (torch.randn(n, K, device="cuda").bfloat16() for n in (M, N))
+    x, y = torch.empty(M, N, device="cuda", dtype=torch.bfloat16), torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    E.gemm(a, b, x, False, True, False)
+    E.gemm_pair(a, b, y, False, True, False)
+    assert torch.equal(x, y)
