@@ -16,8 +16,8 @@ int mt_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const float
 int mt_rmsnorm_bwd_partial_rows(int rows, int D, int sms);
 int mt_rope(void* x, const int* pos, const float* inv_ts, long tokens, int heads, int dh, int n_rot, int rot_dim, int interleaved,
             int inverse, cudaStream_t st);
-int mt_gated_act_fwd(const void* gu, void* out, long rows, int F, int code, int sms, cudaStream_t st);
-int mt_gated_act_bwd(const void* dy, const void* gu, void* dgu, long rows, int F, int code, int sms, cudaStream_t st);
+int mt_gated_act_fwd(const void* gu, void* out, long rows, int F, int code, cudaStream_t st);
+int mt_gated_act_bwd(const void* dy, const void* gu, void* dgu, long rows, int F, int code, cudaStream_t st);
 int mt_embedding_fwd(const int* tok, const void* table, void* out, long tokens, int D, int V, cudaStream_t st);
 int mt_embedding_bwd(const int* tok, const void* dy, float* dtable, long tokens, int D, int V, cudaStream_t st);
 int mt_xent(void* logits, const int* targets, const float* weights, float z_loss, float* loss_out, float* z_out, long rows, long ld,
@@ -250,13 +250,13 @@ void rope_inplace(torch::Tensor& x, const torch::Tensor& pos, const torch::Tenso
 void gated_act_fwd(const torch::Tensor& gu, torch::Tensor& out, int64_t code) {
   TORCH_CHECK(gu.is_contiguous() && out.is_contiguous() && gu.size(1) == 2 * out.size(1));
   c10::cuda::CUDAGuard guard(gu.device());
-  check(mt_gated_act_fwd(gu.data_ptr(), out.data_ptr(), gu.size(0), (int)out.size(1), (int)code, num_sms(), cur_stream()), "gated_act_fwd");
+  check(mt_gated_act_fwd(gu.data_ptr(), out.data_ptr(), gu.size(0), (int)out.size(1), (int)code, cur_stream()), "gated_act_fwd");
 }
 
 void gated_act_bwd(const torch::Tensor& dy, const torch::Tensor& gu, torch::Tensor& dgu, int64_t code) {
   TORCH_CHECK(gu.is_contiguous() && dy.is_contiguous() && dgu.is_contiguous());
   c10::cuda::CUDAGuard guard(gu.device());
-  check(mt_gated_act_bwd(dy.data_ptr(), gu.data_ptr(), dgu.data_ptr(), gu.size(0), (int)dy.size(1), (int)code, num_sms(), cur_stream()),
+  check(mt_gated_act_bwd(dy.data_ptr(), gu.data_ptr(), dgu.data_ptr(), gu.size(0), (int)dy.size(1), (int)code, cur_stream()),
         "gated_act_bwd");
 }
 

@@ -189,3 +189,63 @@ def test_muon_newton_schulz_on_the_repository_gemm():
     assert (got - want).abs().max() < 0.05 * want.abs().max() + 0.02, (got - want).abs().max()
     sv = torch.linalg.svdvals(got)
     assert float(sv.max()) < 1.3 and float(sv.min()) > 0.4
+
+
+@pytest.mark.parametrize("rows,F", [(1, 8), (2, 2048), (3, 2056), (131, 4104)])
+@pytest.mark.parametrize("code", [0, 1, 2, 3])
+def test_gated_act_edges(rows, F, code):
+  """Odd row counts and widths around a block's 2048 columns: every element within two bf16 ulps of fp64 (one for the result, one for the exponential
+  and the products in fp32 far below it)."""
+  E = _E()
+  g = torch.Generator(device="cuda").manual_seed(F)
+  gu, dy = (torch.randn(rows, n * F, device="cuda", generator=g).bfloat16() for n in (2, 1))
+  out, dgu = torch.empty_like(dy), torch.empty_like(gu)
+  E.gated_act_fwd(gu, out, code)
+  E.gated_act_bwd(dy, gu, dgu, code)
+  x = gu.double().requires_grad_(True)
+  f = {0: torch.nn.functional.silu, 1: lambda t: torch.nn.functional.gelu(t, approximate="tanh"), 2: torch.relu, 3: lambda t: t}[code]
+  want = f(x[:, :F]) * x[:, F:]
+  want.backward(dy.double())
+  for a, b in ((out, want.detach()), (dgu, x.grad)):
+    assert bool(((a.double() - b).abs() <= 2 ** -8 * b.abs() + 1e-5).all())
+
+
+@pytest.mark.parametrize("heads,n_rot,dh,rot", [(1, 1, 16, 16), (5, 3, 64, 32), (40, 40, 128, 128), (33, 32, 256, 128), (3, 3, 24, 24), (4, 4, 80, 40)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_rope_widths(heads, n_rot, dh, rot, interleaved):
+  """Rotated widths that the 16-byte kernel takes and widths that it leaves to the other one; lanes and heads that are not rotated stay the same bits.
+  The reference rounds its angles and products in fp32 too: one bf16 ulp of the larger lane of a pair apart at most."""
+  E = _E()
+  B, S = 2, 37
+  x = torch.randn(B, S, heads, dh, device="cuda").bfloat16()
+  pos = (torch.arange(S, device="cuda", dtype=torch.int32)[None] * 7 + 1).expand(B, S).contiguous()
+  inv = ref.rope_inv_timescale(rot, 1, 10000).cuda()
+  for inverse in (False, True):
+    y = x.clone()
+    E.rope_inplace(y.view(B * S, heads, dh), pos.reshape(-1), inv, n_rot, interleaved, inverse, rot)
+    want = ref.apply_rope(x[:, :, :n_rot], pos, inv, interleaved, rot, inverse).float()
+    assert bool(((y[:, :, :n_rot].float() - want).abs() <= 2 ** -7 * want.abs() + 2 ** -7).all())
+    assert torch.equal(y[:, :, n_rot:], x[:, :, n_rot:]) and torch.equal(y[..., rot:], x[..., rot:])
+
+
+@pytest.mark.parametrize("V", [8, 100, 8191, 8200, 32003, 151936])
+def test_cross_entropy_widths(V):
+  """Widths around one and two vectors per thread and with a tail, logits with -inf among them. loss within 2**-20 of the log-sum-exp's size of fp64 (fp32
+  sums of at most 40 terms per thread); gradients within one bf16 ulp."""
+  E = _E()
+  g = torch.Generator(device="cuda").manual_seed(V)
+  rows, ld = 5, (V + 7) // 8 * 8
+  store = (torch.randn(rows, ld, device="cuda", generator=g) * 4).bfloat16()
+  store[1, 3: V: 5] = float("-inf")
+  tgt = torch.tensor([0, 1, V - 1, V // 2, 7], device="cuda", dtype=torch.int32)
+  wt = torch.tensor([1.0, 0.5, 1.0, 0.0, 2.0], device="cuda")
+  lg = store[:, :V].double()
+  lse = torch.logsumexp(lg, -1)
+  want = lse - lg.gather(1, tgt.long()[:, None])[:, 0]
+  grad = wt.double()[:, None] * (torch.softmax(lg, -1) - torch.nn.functional.one_hot(tgt.long(), V))
+  work = store.clone()
+  loss, z = torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda")
+  E.xent_fwd_bwd(work[:, :V], tgt, wt, 0.0, loss, z, True)
+  assert bool(((loss.double() - want).abs() <= 2 ** -20 * (lse.abs() + want.abs() + 1)).all())
+  assert bool(((work[:, :V].double() - grad).abs() <= 2 ** -8 * grad.abs() + 1e-6).all())
+  assert torch.equal(work[:, V:], store[:, V:])
