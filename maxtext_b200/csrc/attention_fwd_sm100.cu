@@ -163,7 +163,7 @@ __device__ __forceinline__ void flash_fwd_body(const CUtensorMap& map_q, const C
 
   if (warp == 0) {
     // ================================================================ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_arrive_expect_tx(bar(Q_FULL), NQ * QT);
 #pragma unroll
       for (int i = 0; i < NQ; ++i)
@@ -185,7 +185,7 @@ __device__ __forceinline__ void flash_fwd_body(const CUtensorMap& map_q, const C
     }
   } else if (warp == 1) {
     // ================================================================ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(128, DV, false, true);
       int cnt[NQ];

@@ -91,7 +91,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -109,7 +109,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_fp8(BM, BN, 0, 0);
       int s = 0, acc = 0;
       uint32_t ph = 0, aph = 0;

@@ -268,7 +268,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   } else if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one thread)
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -305,7 +305,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = FP8 ? make_idesc_fp8(BM, BN, (uint32_t)p.q_fmt_a, (uint32_t)p.q_fmt_b) : make_idesc_bf16(BM, BN, A_MN, B_MN);
       constexpr uint32_t A_LBO = A_MN ? 8192 : 16, B_LBO = B_MN ? 8192 : 16;
       constexpr uint32_t A_KSTEP = A_MN ? 2048 : 32, B_KSTEP = B_MN ? 2048 : 32;  // bytes per UMMA_K
@@ -833,7 +833,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one thread per CTA)
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -866,7 +866,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (one thread of the leader CTA)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = FP8 ? make_idesc_fp8(2 * BM, BN, (uint32_t)p.q_fmt_a, (uint32_t)p.q_fmt_b) : make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       constexpr uint32_t A_LBO = A_MN ? 8192 : 16, B_LBO = B_MN ? 8192 : 16;
       constexpr uint32_t A_KSTEP = A_MN ? 2048 : 32, B_KSTEP = B_MN ? 2048 : 32;
