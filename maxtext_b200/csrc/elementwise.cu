@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
 // in a fixed order: no atomics, so the result is bitwise reproducible.
 // As in the forward pass the next row is fetched before the present one is summed: 110 us for 16384 x 4096 with a stream gradient (537 MB), 192 us without.
 template <int TPR, int VPT>
-__global__ void __launch_bounds__(256, VPT == 1 ? 3 : VPT == 2 ? 2 : 1) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256, TPR == 32 ? (VPT == 1 ? 4 : 1) : VPT == 1 ? 3 : VPT == 2 ? 2 : 1) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                    const __nv_bfloat16* __restrict__ scale, const float* __restrict__ rstd_in, float offset,
                                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows,
                                    int D) {
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256, VPT == 1 ? 3 : VPT == 2 ? 2 : 1) rmsnorm_
 #pragma unroll
     for (int e = 0; e < 8; ++e) ds[i][e] = 0.f;
   const long n_groups = ((long)rows + rows_per_block - 1) / rows_per_block;
-  constexpr bool AHEAD = VPT <= 2;                           // wider rows have no registers left for it
+  constexpr bool AHEAD = TPR == 256 && VPT <= 2;             // a warp per row has enough rows under way; wider rows have no registers left for it
   bf16x8 nd[VPT], nx[VPT];                                   // the next row
   float nrstd = 0.f;
   auto fetch = [&](long grp) {
