@@ -40,8 +40,10 @@ def _small_m_wins(M, N, K) -> bool:
   weights at M <= 32: 11.4 - 15.3 us against 15.6 - 17.1 us). Its mma.sync inner loop runs out of issue rate above M = 32, and
   on wider or deeper weights the library's kernels are ahead, so those go to the library (and are counted as fallbacks).
   MAXTEXT_B200_SMALL_M=all / none overrides the rule."""
+  if M > 64:
+    return False
   mode = os.environ.get("MAXTEXT_B200_SMALL_M", "")
-  if mode == "none" or M > 64:
+  if mode == "none":
     return False
   if mode == "all":
     return True
@@ -182,9 +184,10 @@ def linear(x: torch.Tensor, p, saved_out: torch.Tensor | None = None, bias=None,
   if not torch.is_grad_enabled():
     if saved_out is not None:
       return saved_out
-    y = (pre if pre is not None else _quant.block_linear_fwd(x2, p.data) if _quant.block_supported(x2, p.data) else
-         _quant.int8_linear_fwd(x2, p.data) if _quant.int8_on() else
-         (_quant.linear_fwd(x2, p.data, p) if _quant.supported(x2, p.data) else mm(x2, p.data, False, True)))
+    w = p.data if pre is None else None          # read once: a fused parameter checks its parts each time
+    y = (pre if pre is not None else _quant.block_linear_fwd(x2, w) if _quant.block_supported(x2, w) else
+         _quant.int8_linear_fwd(x2, w) if _quant.int8_on() else
+         (_quant.linear_fwd(x2, w, p) if _quant.supported(x2, w) else mm(x2, w, False, True)))
     if lo is not None:
       y = y + _lora_delta(x2, lo).to(y.dtype)
     y = y.view(*x.shape[:-1], p.shape[0])
