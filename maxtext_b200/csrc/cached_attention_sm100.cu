@@ -416,9 +416,9 @@ struct DecodeArgs {
   float *part, *ml;                    // part [B, H, splits, Dv], ml [B, H, splits, 2]
 };
 
-constexpr int KEYS = 16, RING = 3;     // keys of a warp's tile, tiles in flight
+constexpr int KEYS = 16;               // keys of a warp's tile
 
-template <int DK, int DVT>             // widths rounded up to the template: DK, DVT multiples of 16
+template <int DK, int DVT, int RING>   // widths rounded up to the template: DK, DVT multiples of 16; RING - 1 tiles in flight per warp
 __global__ void __launch_bounds__(128)
 decode_kernel(const DecodeArgs a) {
   constexpr int LK = DK + 8, LV = DVT + 8, TILE = KEYS * (LK + LV);
@@ -1160,14 +1160,33 @@ int prep_t(const PrepArgs& a, long N, cudaStream_t st) {
   return a.talk ? pick(std::true_type{}) : pick(std::false_type{});
 }
 
-template <int DK, int DVT>
-int decode_run(const DecodeArgs& a, int B, cudaStream_t st) {
+template <int DK, int DVT, int RING>
+int decode_ring(const DecodeArgs& a, int B, cudaStream_t st) {
   constexpr int ring = (16 * (DK + 8) + 4 * RING * KEYS * (DK + 8 + DVT + 8)) * 2, join = 4 * 16 * (DVT + 4) * 4;
   constexpr int smem = ring > join ? ring : join;
-  auto k = decode_kernel<DK, DVT>;
+  auto k = decode_kernel<DK, DVT, RING>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
   k<<<dim3(a.splits, a.G * a.head_blocks, B), 128, smem, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+// Two or three tiles of a warp in shared memory. Heads of 128 lanes let three CTAs share an SM with two tiles, two CTAs with three. A warp's chain of
+// tiles (matrix instructions with two to sixteen rows in use) is what bounds a CTA, and a wave of one, two or three CTAs per SM takes 40, 48 or 72 us at 1500
+// keys (5 : 6 : 9), whichever the number of tiles; so the count of CTAs decides. With two tiles: 360 CTAs 73 us against 93 with three, 2048 CTAs (128 slots, 2048
+// keys) 198 against 214; with three: 480 CTAs 97 us against 114. Other widths keep three tiles.
+bool two_tiles(long ctas) {
+  constexpr long SMS = 148, T[4] = {0, 5, 6, 9};
+  auto cost = [&](long per_sm) {
+    const long wave = per_sm * SMS, rest = ctas % wave;
+    return ctas / wave * T[per_sm] + T[(rest + SMS - 1) / SMS];
+  };
+  return cost(3) <= cost(2);
+}
+template <int DK, int DVT>
+int decode_run(const DecodeArgs& a, int B, cudaStream_t st) {
+  if constexpr (DK == 128 && DVT == 128) {
+    if (two_tiles((long)a.splits * a.G * a.head_blocks * B)) return decode_ring<DK, DVT, 2>(a, B, st);
+  }
+  return decode_ring<DK, DVT, 3>(a, B, st);
 }
 template <int DK>
 int decode_dv(const DecodeArgs& a, int B, cudaStream_t st) {

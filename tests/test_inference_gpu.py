@@ -126,3 +126,26 @@ def test_one_kernel_for_q_k_v_and_the_cache_matches_the_separate_ones(name, head
     for n in ("k", "v"):
       x, y = getattr(a[0], n).float(), getattr(b[0], n).float()
       assert torch.equal(x == 0, y == 0) and float((x - y).norm() / x.norm()) <= 2 ** -5
+
+
+def test_decode_attention_is_the_same_bits_however_many_ctas_share_an_sm():
+  """45 sequences (360 CTAs) run with two tiles per warp in shared memory, 60 (480) with three: every sequence's result depends on its own keys only."""
+  from maxtext_b200.ops import backend
+  E = backend.ext(required=True)
+  g = torch.Generator(device="cuda").manual_seed(0)
+  B, H, G, D, L = 60, 16, 8, 128, 200
+  k, v = (torch.randn(B, L, G, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+  q = torch.randn(B, H, D, device="cuda", generator=g).bfloat16()
+  ln = torch.randint(1, L - 1, (B,), device="cuda", generator=g)
+
+  def run(n):
+    part, ml = torch.empty(n, H, 1, D, device="cuda"), torch.empty(n, H, 1, 2, device="cuda")
+    out = torch.empty(n, H * D, device="cuda", dtype=torch.bfloat16)
+    E.cached_decode(q[:n].contiguous(), k, v, torch.arange(n, device="cuda"), ln[:n].contiguous(), 0.1, 0.0, 0, None, None, 1, part, ml, out)
+    return out
+  few, many = run(45), run(60)
+  assert torch.equal(few, many[:45])
+  b, n = 7, int(ln[7]) + 1
+  s = torch.softmax(torch.einsum("gjd,ngd->gjn", q[b].view(G, 2, D).double(), k[b, :n].double()) * 0.1, -1)
+  want = torch.einsum("gjn,ngd->gjd", s, v[b, :n].double()).reshape(-1)
+  assert bool(((few[b].double() - want).abs() <= 2 ** -7 * want.abs().max()).all())
