@@ -18,6 +18,9 @@ int mt_rope(void* x, const int* pos, const float* inv_ts, long tokens, int heads
             int inverse, cudaStream_t st);
 int mt_gated_act_fwd(const void* gu, void* out, long rows, int F, int code, cudaStream_t st);
 int mt_gated_act_bwd(const void* dy, const void* gu, void* dgu, long rows, int F, int code, cudaStream_t st);
+int mt_latent_heads_ok(int nope, int rope, int vd, int paired);
+int mt_latent_heads(int backward, const void* in0, const void* in1, const void* in2, void* out0, void* out1, void* out2, const int* pos, const float* inv_ts,
+                    long tokens, int H, int nope, int rope, int vd, long ldkr, float scale, int paired, cudaStream_t st);
 int mt_embedding_fwd(const int* tok, const void* table, void* out, long tokens, int D, int V, cudaStream_t st);
 int mt_embedding_bwd(const int* tok, const void* dy, float* dtable, long tokens, int D, int V, cudaStream_t st);
 int mt_xent(void* logits, const int* targets, const float* weights, float z_loss, float* loss_out, float* z_out, long rows, long ld,
@@ -260,6 +263,29 @@ void gated_act_bwd(const torch::Tensor& dy, const torch::Tensor& gu, torch::Tens
         "gated_act_bwd");
 }
 
+// forward: (q [N, H, nope + rope], kr [N, rope] rows of any stride, kv [N, H, nope + vd]) -> (qo, k [N, H, nope + rope], v [N, H, vd])
+// backward: (dqo, dk, dv) -> (dq, dkr, dkv), all contiguous
+void latent_heads(bool backward, const torch::Tensor& in0, const torch::Tensor& in1, const torch::Tensor& in2, torch::Tensor& out0, torch::Tensor& out1,
+                  torch::Tensor& out2, const torch::Tensor& pos, const torch::Tensor& inv_ts, int64_t nope, double scale, bool paired) {
+  const torch::Tensor &kr = backward ? out1 : in1, &v = backward ? in2 : out2, &q = in0;
+  TORCH_CHECK(q.is_cuda() && q.dim() == 3 && kr.dim() == 2 && v.dim() == 3 && kr.stride(1) == 1);
+  const int64_t N = q.size(0), H = q.size(1), rope = kr.size(1), vd = v.size(2);
+  TORCH_CHECK(q.size(2) == nope + rope && kr.size(0) == N && mt_latent_heads_ok((int)nope, (int)rope, (int)vd, paired));
+  const torch::Tensor *t[6] = {&in0, &in1, &in2, &out0, &out1, &out2};
+  const int64_t qn = N * H * (nope + rope), kvn = N * H * (nope + vd), vn = N * H * vd;
+  const int64_t want[6] = {qn, backward ? qn : N * rope, backward ? vn : kvn, qn, backward ? N * rope : qn, backward ? kvn : vn};
+  for (int i = 0; i < 6; ++i)
+    TORCH_CHECK(t[i]->is_cuda() && t[i]->scalar_type() == torch::kBFloat16 && t[i]->numel() == want[i] && reinterpret_cast<uintptr_t>(t[i]->data_ptr()) % 16 == 0 &&
+                    (t[i]->is_contiguous() || (!backward && i == 1 && kr.stride(0) % 8 == 0)),
+                "latent_heads: operand ", i);
+  TORCH_CHECK(pos.scalar_type() == torch::kInt32 && pos.is_contiguous() && pos.numel() == N && inv_ts.scalar_type() == torch::kFloat32 &&
+              inv_ts.is_contiguous() && inv_ts.numel() == rope / 2);
+  c10::cuda::CUDAGuard guard(q.device());
+  check(mt_latent_heads(backward, in0.data_ptr(), in1.data_ptr(), in2.data_ptr(), out0.data_ptr(), out1.data_ptr(), out2.data_ptr(), pos.data_ptr<int>(),
+                        inv_ts.data_ptr<float>(), N, (int)H, (int)nope, (int)rope, (int)vd, kr.stride(0), (float)scale, paired, cur_stream()),
+        "mt_latent_heads");
+}
+
 void embedding_fwd(const torch::Tensor& tok, const torch::Tensor& table, torch::Tensor& out) {
   TORCH_CHECK(tok.scalar_type() == torch::kInt32 && table.is_contiguous() && out.is_contiguous());
   c10::cuda::CUDAGuard guard(table.device());
@@ -339,6 +365,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rope_inplace", &rope_inplace);
   m.def("gated_act_fwd", &gated_act_fwd);
   m.def("gated_act_bwd", &gated_act_bwd);
+  m.def("latent_heads", &latent_heads);
+  m.def("latent_heads_ok", [](int64_t nope, int64_t rope, int64_t vd, bool paired) { return mt_latent_heads_ok((int)nope, (int)rope, (int)vd, paired) != 0; });
   m.def("embedding_fwd", &embedding_fwd);
   m.def("embedding_bwd", &embedding_bwd);
   register_attention(m);

@@ -497,6 +497,146 @@ __global__ void embedding_bwd_kernel(const int* __restrict__ tok, const __nv_bfl
   for (int i = threadIdx.x; i < D; i += blockDim.x) atomicAdd(dtable + (long)id * D + i, __bfloat162float(dy[t * D + i]));
 }
 
+// ------------------------------------------------------------------------------------------------ heads of latent attention
+// What latent attention does between its projections and the attention kernel, in one pass over a token:
+//   q [H, nope + rope] -> [q_nope | rot(q_rope)] * scale;   k = [kv_nope | rot(kr) for every head];   v = the rest of kv [H, nope + vd]
+// with the roundings of the separate steps (after the rotation and after the scale), and the way back: dkr sums over the heads. Bandwidth-bound: a thread
+// moves 16-byte columns (rotated ones in pairs). As rotations, concatenations, products, copies and their zero-filled gradients it was about 70 launches and
+// 1.0 ms of a training step of two layers at 4096 tokens (16 heads of 128 + 64 and 128); six launches of 41 us now.
+struct LatentHeads {
+  int H, nope, rope, vd;
+  long ldkr;                            // row stride of kr
+  float scale;
+  const int* pos;
+  const float* inv_ts;
+};
+__device__ __forceinline__ bf16x8 scaled8(const bf16x8& p, float scale) {
+  float f[8];
+  unpack8(p, f);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) f[e] *= scale;
+  return pack8(f);
+}
+// lanes j .. j + 7 of a rotated row (PAIRED: neighbours turn together; otherwise lane j with lane j + rope / 2, and `b` holds the second ones)
+template <bool PAIRED>
+__device__ __forceinline__ void turn8(const float2* cs, int j, bf16x8& a, bf16x8& b) {
+  float x[8], y[8], o[8], t[8];
+  unpack8(a, x);
+  if (PAIRED) {
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      const float2 c = cs[(j + e) / 2];
+      o[e] = __fmaf_rn(x[e], c.x, -__fmul_rn(x[e + 1], c.y));
+      o[e + 1] = __fmaf_rn(x[e], c.y, __fmul_rn(x[e + 1], c.x));
+    }
+    a = pack8(o);
+  } else {
+    unpack8(b, y);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float2 c = cs[j + e];
+      o[e] = __fmaf_rn(x[e], c.x, -__fmul_rn(y[e], c.y));
+      t[e] = __fmaf_rn(x[e], c.y, __fmul_rn(y[e], c.x));
+    }
+    a = pack8(o);
+    b = pack8(t);
+  }
+}
+__device__ __forceinline__ bf16x8 ld8(const __nv_bfloat16* p) { return *reinterpret_cast<const bf16x8*>(p); }
+__device__ __forceinline__ void st8(__nv_bfloat16* p, const bf16x8& v) { *reinterpret_cast<bf16x8*>(p) = v; }
+
+template <bool PAIRED>
+__global__ void __launch_bounds__(256) latent_heads_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kr,
+                                                               const __nv_bfloat16* __restrict__ kv, __nv_bfloat16* __restrict__ qo,
+                                                               __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ v, const LatentHeads a) {
+  extern __shared__ __align__(16) float2 cs[];
+  const long n = blockIdx.x;
+  const int half = a.rope / 2, qk = a.nope + a.rope, kvw = a.nope + a.vd;
+  const float p = (float)a.pos[n];
+  for (int j = threadIdx.x; j < half; j += blockDim.x) {
+    float s, c;
+    sincosf(p * a.inv_ts[j], &s, &c);
+    cs[j] = make_float2(c, s);
+  }
+  __syncthreads();
+  const int un = a.nope / 8, ur = (PAIRED ? a.rope : half) / 8, uv = a.vd / 8, per = un + ur + uv;
+  for (int i = threadIdx.x; i < a.H * per; i += blockDim.x) {
+    const int h = i / per, u = i % per;
+    const __nv_bfloat16 *qh = q + (n * a.H + h) * qk, *kvh = kv + (n * a.H + h) * kvw;
+    __nv_bfloat16 *qoh = qo + (n * a.H + h) * qk, *kh = k + (n * a.H + h) * qk;
+    if (u < un) {
+      st8(qoh + u * 8, scaled8(ld8(qh + u * 8), a.scale));
+      st8(kh + u * 8, ld8(kvh + u * 8));
+    } else if (u < un + ur) {
+      const int j = (u - un) * 8;
+      bf16x8 x = ld8(qh + a.nope + j), y, r = ld8(kr + n * a.ldkr + j), t;
+      if (!PAIRED) { y = ld8(qh + a.nope + j + half); t = ld8(kr + n * a.ldkr + j + half); }
+      turn8<PAIRED>(cs, j, x, y);
+      turn8<PAIRED>(cs, j, r, t);
+      st8(qoh + a.nope + j, scaled8(x, a.scale));
+      st8(kh + a.nope + j, r);
+      if (!PAIRED) {
+        st8(qoh + a.nope + j + half, scaled8(y, a.scale));
+        st8(kh + a.nope + j + half, t);
+      }
+    } else {
+      const int j = (u - un - ur) * 8;
+      st8(v + (n * a.H + h) * a.vd + j, ld8(kvh + a.nope + j));
+    }
+  }
+}
+
+template <bool PAIRED>
+__global__ void __launch_bounds__(256) latent_heads_bwd_kernel(const __nv_bfloat16* __restrict__ dqo, const __nv_bfloat16* __restrict__ dk,
+                                                               const __nv_bfloat16* __restrict__ dv, __nv_bfloat16* __restrict__ dq,
+                                                               __nv_bfloat16* __restrict__ dkr, __nv_bfloat16* __restrict__ dkv, const LatentHeads a) {
+  extern __shared__ __align__(16) float2 cs[];
+  const long n = blockIdx.x;
+  const int half = a.rope / 2, qk = a.nope + a.rope, kvw = a.nope + a.vd;
+  __nv_bfloat16* sum = reinterpret_cast<__nv_bfloat16*>(cs + half);          // [rope]
+  const float p = (float)a.pos[n];
+  for (int j = threadIdx.x; j < half; j += blockDim.x) {
+    float s, c;
+    sincosf(p * a.inv_ts[j], &s, &c);
+    cs[j] = make_float2(c, -s);
+  }
+  for (int j = threadIdx.x; j < a.rope; j += blockDim.x) {
+    float t = 0.f;
+    for (int h = 0; h < a.H; ++h) t += __bfloat162float(dk[(n * a.H + h) * qk + a.nope + j]);
+    sum[j] = __float2bfloat16_rn(t);
+  }
+  __syncthreads();
+  const int un = a.nope / 8, ur = (PAIRED ? a.rope : half) / 8, uv = a.vd / 8, per = un + ur + uv;
+  for (int i = threadIdx.x; i < a.H * per + ur; i += blockDim.x) {
+    const int h = i / per, u = i % per;
+    if (h == a.H) {                                          // the shared rotated key
+      const int j = u * 8;
+      bf16x8 x = ld8(sum + j), y;
+      if (!PAIRED) y = ld8(sum + j + half);
+      turn8<PAIRED>(cs, j, x, y);
+      st8(dkr + n * a.rope + j, x);
+      if (!PAIRED) st8(dkr + n * a.rope + j + half, y);
+      continue;
+    }
+    const __nv_bfloat16 *gq = dqo + (n * a.H + h) * qk, *gk = dk + (n * a.H + h) * qk;
+    __nv_bfloat16 *oq = dq + (n * a.H + h) * qk, *okv = dkv + (n * a.H + h) * kvw;
+    if (u < un) {
+      st8(oq + u * 8, scaled8(ld8(gq + u * 8), a.scale));
+      st8(okv + u * 8, ld8(gk + u * 8));
+    } else if (u < un + ur) {
+      const int j = (u - un) * 8;
+      bf16x8 x = scaled8(ld8(gq + a.nope + j), a.scale), y;
+      if (!PAIRED) y = scaled8(ld8(gq + a.nope + j + half), a.scale);
+      turn8<PAIRED>(cs, j, x, y);
+      st8(oq + a.nope + j, x);
+      if (!PAIRED) st8(oq + a.nope + j + half, y);
+    } else {
+      const int j = (u - un - ur) * 8;
+      st8(okv + a.nope + j, ld8(dv + (n * a.H + h) * a.vd + j));
+    }
+  }
+}
+
 }  // namespace mt
 
 // ================================================================================================ launchers
@@ -611,5 +751,24 @@ extern "C" int mt_embedding_fwd(const int* tok, const void* table, void* out, lo
 extern "C" int mt_embedding_bwd(const int* tok, const void* dy, float* dtable, long tokens, int D, int V, cudaStream_t st) {
   if (tokens <= 0) return 0;
   embedding_bwd_kernel<<<(unsigned)tokens, 256, 0, st>>>(tok, (const __nv_bfloat16*)dy, dtable, D, V);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+// Widths in multiples of 8 (rotated halves too), pointers and the row stride of kr aligned to 16 bytes.
+extern "C" int mt_latent_heads_ok(int nope, int rope, int vd, int paired) {
+  return nope > 0 && rope > 0 && vd > 0 && nope % 8 == 0 && vd % 8 == 0 && rope % (paired ? 8 : 16) == 0 && rope <= 2048;
+}
+
+// backward 0: q, kr, kv -> qo, k, v.  backward 1: dqo, dk, dv -> dq, dkr [tokens, rope], dkv.
+extern "C" int mt_latent_heads(int backward, const void* in0, const void* in1, const void* in2, void* out0, void* out1, void* out2, const int* pos,
+                               const float* inv_ts, long tokens, int H, int nope, int rope, int vd, long ldkr, float scale, int paired, cudaStream_t st) {
+  if (!mt_latent_heads_ok(nope, rope, vd, paired) || H < 1 || ldkr % 8) return -1;
+  if (tokens <= 0) return 0;
+  const LatentHeads a{H, nope, rope, vd, ldkr, scale, pos, inv_ts};
+  const int smem = rope / 2 * (int)sizeof(float2) + rope * 2;
+  using B = __nv_bfloat16;
+  auto k = backward ? (paired ? latent_heads_bwd_kernel<true> : latent_heads_bwd_kernel<false>)
+                    : (paired ? latent_heads_fwd_kernel<true> : latent_heads_fwd_kernel<false>);
+  k<<<(unsigned)tokens, 256, smem, st>>>((const B*)in0, (const B*)in1, (const B*)in2, (B*)out0, (B*)out1, (B*)out2, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

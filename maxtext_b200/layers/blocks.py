@@ -680,16 +680,10 @@ class MLA:
       low_rank_q = self.q_norm(F.linear(x, self.wq_a))
       q = F.linear(low_rank_q, self.wq_b)
     q = q.view(B, S, self.h, self.qk)
-    q_nope, q_rope = q[..., :self.nope], q[..., self.nope:]
-    q_rope = F.rope(q_rope, ctx.positions, self.inv_ts, self.interleaved)
-    q = torch.cat([q_nope, q_rope], dim=-1) * self.softmax_scale
     kva = F.linear(x, self.wkv_a)
-    latent, k_rope = kva[..., :self.kv_rank], kva[..., self.kv_rank:]
-    k_rope = F.rope(k_rope.reshape(B, S, 1, self.rope_d), ctx.positions, self.inv_ts, self.interleaved)
-    latent = self.kv_norm(latent.contiguous())
+    latent = self.kv_norm(kva[..., :self.kv_rank].contiguous())
     kv = F.linear(latent, self.wkv_b).view(B, S, self.h, self.nope + self.vd)
-    k = torch.cat([kv[..., :self.nope], k_rope.expand(B, S, self.h, self.rope_d)], dim=-1)
-    v = kv[..., self.nope:]
+    q, k, v = F.latent_heads(q, kva[..., self.kv_rank:], kv, ctx.positions, self.inv_ts, self.nope, self.softmax_scale, self.interleaved)
     if c.use_qk_clip and ctx.mode == "train" and not ctx.recompute and ctx.max_logits is not None:
       ctx.max_logits[(ctx.layer_index, self)] = _max_logit_per_head(q, k, ctx.positions, ctx.segment_ids)
     sparse = None

@@ -832,6 +832,46 @@ class _RopeFn(torch.autograd.Function):
     return rope_packed_(dx, positions, inv_ts, dx.shape[2], interleaved, True, rotary_dim), None, None, None, None
 
 
+class _LatentHeadsFn(torch.autograd.Function):
+  @staticmethod
+  def forward(ctx, q, kr, kv, pos, inv_ts, nope, scale, interleaved):
+    N, H, qk = q.shape
+    ctx.save_for_backward(pos, inv_ts)
+    ctx.cfg = (nope, scale, interleaved, kr.shape[1], kv.shape[2])
+    qo, k, v = torch.empty_like(q), torch.empty_like(q), torch.empty(N, H, kv.shape[2] - nope, dtype=q.dtype, device=q.device)
+    backend.ext().latent_heads(False, q, kr, kv, qo, k, v, pos, inv_ts, nope, scale, interleaved)
+    return qo, k, v
+
+  @staticmethod
+  def backward(ctx, dqo, dk, dv):
+    pos, inv_ts = ctx.saved_tensors
+    nope, scale, interleaved, rope_d, kvw = ctx.cfg
+    N, H, _ = dqo.shape
+    dq, dkr = torch.empty_like(dqo, memory_format=torch.contiguous_format), torch.empty(N, rope_d, dtype=dqo.dtype, device=dqo.device)
+    dkv = torch.empty(N, H, kvw, dtype=dqo.dtype, device=dqo.device)
+    backend.ext().latent_heads(True, dqo.contiguous(), dk.contiguous(), dv.contiguous(), dq, dkr, dkv, pos, inv_ts, nope, scale, interleaved)
+    return dq, dkr, dkv, None, None, None, None, None
+
+
+def latent_heads(q, k_rope, kv, positions, inv_ts, nope, scale, interleaved=False):
+  """Queries, keys and values of latent attention from its projections: q [B, S, H, nope + rope] -> its last lanes rotated, all times `scale`;
+  k_rope [B, S, rope], rotated, behind every head's first `nope` lanes of kv [B, S, H, nope + vd]; the rest of kv. On a GPU one kernel per pass."""
+  B, S, H, qk = q.shape
+  rope_d, kvw = k_rope.shape[-1], kv.shape[-1]
+  if (backend.use_cuda_kernels(q) and q.dtype == k_rope.dtype == kv.dtype == torch.bfloat16 and q.is_contiguous() and kv.is_contiguous()
+      and qk == nope + rope_d and inv_ts.dtype == torch.float32 and inv_ts.is_contiguous() and inv_ts.numel() == rope_d // 2
+      and positions.numel() == B * S and k_rope.stride(-1) == 1 and k_rope.stride(-2) % 8 == 0 and (B == 1 or k_rope.stride(0) == S * k_rope.stride(1))
+      and all(t.data_ptr() % 16 == 0 for t in (q, k_rope, kv)) and backend.ext().latent_heads_ok(nope, rope_d, kvw - nope, bool(interleaved))):
+    pos = positions.reshape(-1).to(torch.int32).contiguous()
+    args = (q.view(B * S, H, qk), k_rope.reshape(B * S, rope_d), kv.view(B * S, H, kvw), pos, inv_ts, int(nope), float(scale), bool(interleaved))
+    qo, k, v = _LatentHeadsFn.apply(*args) if torch.is_grad_enabled() else _LatentHeadsFn.forward(_Dummy(), *args)
+    return qo.view(q.shape), k.view(q.shape), v.view(B, S, H, kvw - nope)
+  q = torch.cat([q[..., :nope], rope(q[..., nope:], positions, inv_ts, interleaved)], dim=-1) * scale
+  kr = rope(k_rope.reshape(B, S, 1, rope_d), positions, inv_ts, interleaved)
+  k = torch.cat([kv[..., :nope], kr.expand(B, S, H, rope_d)], dim=-1)
+  return q, k, kv[..., nope:]
+
+
 def rope(x, positions, inv_ts, interleaved=False, rotary_dim=None):
   """Out-of-place rotary embedding of x [B,S,H,Dh]."""
   if not torch.is_grad_enabled():

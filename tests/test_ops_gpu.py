@@ -249,3 +249,39 @@ def test_cross_entropy_widths(V):
   assert bool(((loss.double() - want).abs() <= 2 ** -20 * (lse.abs() + want.abs() + 1)).all())
   assert bool(((work[:, :V].double() - grad).abs() <= 2 ** -8 * grad.abs() + 1e-6).all())
   assert torch.equal(work[:, V:], store[:, V:])
+
+
+@pytest.mark.parametrize("B,S,H,nope,rope,vd", [(1, 1, 1, 8, 16, 8), (2, 37, 16, 128, 64, 128), (3, 5, 3, 24, 32, 40), (1, 70, 2, 16, 8, 16), (2, 9, 4, 12, 16, 20)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_latent_heads(B, S, H, nope, rope, vd, interleaved):
+  """The one kernel against the separate steps: the forward pass is the same bits; gradients round once or twice less, and the sum over the heads of
+  the shared key part runs in another order: within two bf16 ulps of the largest addend. Widths that are no multiples of 8 take the separate steps."""
+  from maxtext_b200.ops import functional as F
+  g = torch.Generator(device="cuda").manual_seed(S)
+  rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+  rank = 24
+  q0, kva0, kv0 = rnd(B, S, H, nope + rope), rnd(B, S, rank + rope), rnd(B, S, H, nope + vd)
+  pos = (torch.arange(S, device="cuda")[None] * 3 + torch.arange(B, device="cuda")[:, None])
+  inv = ref.rope_inv_timescale(rope, 1, 10000).cuda()
+  gr = [rnd(B, S, H, nope + rope), rnd(B, S, H, nope + rope), rnd(B, S, H, vd)]
+
+  def run(one):
+    q, kva, kv = (t.clone().requires_grad_(True) for t in (q0, kva0, kv0))
+    kr = kva[..., rank:]
+    if one:
+      out = F.latent_heads(q, kr, kv, pos, inv, nope, 0.07, interleaved)
+    else:
+      k2 = F.rope(kr.reshape(B, S, 1, rope), pos, inv, interleaved)
+      out = (torch.cat([q[..., :nope], F.rope(q[..., nope:], pos, inv, interleaved)], -1) * 0.07,
+             torch.cat([kv[..., :nope], k2.expand(B, S, H, rope)], -1), kv[..., nope:])
+    torch.autograd.backward(out, gr)
+    return out, (q.grad, kva.grad, kv.grad)
+  (o1, g1), (o2, g2) = run(True), run(False)
+  for a, b in zip(o1, o2):
+    assert torch.equal(a, b)
+  with torch.no_grad():
+    for a, b in zip(F.latent_heads(q0, kva0[..., rank:], kv0, pos, inv, nope, 0.07, interleaved), o2):
+      assert torch.equal(a, b)
+  for a, b in zip(g1, g2):
+    assert bool(((a.float() - b.float()).abs() <= 2 ** -7 * b.float().abs() + 2 ** -7 * H).all())
+  assert torch.equal(g1[0], g2[0]) and torch.equal(g1[2], g2[2])
