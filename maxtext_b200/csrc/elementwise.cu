@@ -139,7 +139,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
 
 // ------------------------------------------------------------------------------------------------ RMSNorm backward
 // dx = rstd * (g - xhat * mean(g * xhat)) [+ dres], g = dy * (scale + offset);  dscale += sum_rows dy * xhat. `dres` is what reaches the same row past
-// the norm (the residual stream's own gradient): added here, in fp32, it costs no pass of its own.
+// the norm (the residual stream's own gradient): added here, it costs no pass of its own. It joins the norm's gradient as that is stored (bf16), so the sum
+// is the same bits as of a norm and an add on their own.
 // Blocks stride over rows and keep per-column dscale partials in registers; the warps of a block that work on rows of their own
 // (TPR 32) add theirs up in shared memory, each block writes one row into `partial`, and rms_dscale_reduce_kernel adds the rows up
 // in a fixed order: no atomics, so the result is bitwise reproducible.
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(256, TPR == 32 ? (VPT == 1 ? 4 : 1) : VPT == 1
         if (dres) {
           unpack8(cr[i], a);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) o[e] += a[e];
+          for (int e = 0; e < 8; ++e) o[e] = bf16_round(o[e]) + a[e];
         }
         *reinterpret_cast<bf16x8*>(dx + row * D + col) = pack8(o);
       }

@@ -285,3 +285,21 @@ def test_latent_heads(B, S, H, nope, rope, vd, interleaved):
   for a, b in zip(g1, g2):
     assert bool(((a.float() - b.float()).abs() <= 2 ** -7 * b.float().abs() + 2 ** -7 * H).all())
   assert torch.equal(g1[0], g2[0]) and torch.equal(g1[2], g2[2])
+
+
+def _fma(a, b, c):
+  """a * b + c in fp32, rounded once (the product of two fp32 numbers is exact in fp64)."""
+  return (a.double() * b.double() + c.double()).float()
+
+
+@pytest.mark.parametrize("rows,D", [(1, 8), (4800, 128), (1300, 1032), (2500, 4096), (700, 16384)])
+def test_stream_gradient_is_the_norms_own_plus_the_streams(rows, D):
+  """The norm's gradient joins the stream's as the two would as kernels of their own: rounded, added, rounded. Blocks have several rows."""
+  E = _E()
+  x, dy, dres = (torch.randn(rows, D, device="cuda").bfloat16() for _ in range(3))
+  scale = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16()
+  y, alone, joint, rstd = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x), torch.empty(rows, device="cuda")
+  E.rmsnorm_fwd(x, scale, 1e-5, 0.0, y, rstd)
+  E.rmsnorm_bwd(dy, x, scale, rstd, 0.0, alone, None)
+  E.rmsnorm_bwd(dy, x, scale, rstd, 0.0, joint, None, dres)
+  assert torch.equal(joint, alone + dres)
