@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256, TPR == 32 ? (VPT == 1 ? 4 : 1) : VPT == 1
         unpack8(cx[i], b);
         factor(col, sc);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = rstd * (a[e] * sc[e] - b[e] * rstd * dot);
+        for (int e = 0; e < 8; ++e) o[e] = rstd * __fmaf_rn(-__fmul_rn(b[e], rstd), dot, __fmul_rn(a[e], sc[e]));   // g and xhat rounded as in the sums
         if (dres) {
           unpack8(cr[i], a);
 #pragma unroll

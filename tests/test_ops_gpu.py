@@ -303,3 +303,22 @@ def test_stream_gradient_is_the_norms_own_plus_the_streams(rows, D):
   E.rmsnorm_bwd(dy, x, scale, rstd, 0.0, alone, None)
   E.rmsnorm_bwd(dy, x, scale, rstd, 0.0, joint, None, dres)
   assert torch.equal(joint, alone + dres)
+
+
+def test_norm_gradient_rounds_its_factors_once():
+  """dx of rows of eight lanes, step by step in fp32: g = dy * scale and xhat = x * rstd rounded, their dot product a chain of fused steps,
+  rstd * (g - xhat * mean) with one rounding inside. dy lies near x, so that the difference cancels and every rounding shows; blocks have many rows."""
+  E = _E()
+  rows, D = 400_000, 8
+  x = torch.randn(rows, D, device="cuda").bfloat16()
+  dy = (x.float() + 0.05 * torch.randn(rows, D, device="cuda")).bfloat16()
+  scale = torch.ones(D, device="cuda").bfloat16()
+  rstd = torch.rsqrt(x.float().pow(2).mean(1) + 1e-5)
+  dx = torch.empty_like(x)
+  E.rmsnorm_bwd(dy, x, scale, rstd, 0.25, dx, None)
+  g, xh = dy.float() * 1.25, x.float() * rstd[:, None]
+  dot = torch.zeros(rows, device="cuda")
+  for e in range(D):
+    dot = _fma(g[:, e], xh[:, e], dot)
+  want = rstd[:, None] * _fma(-xh, (dot / D)[:, None].expand_as(xh), g)
+  assert torch.equal(dx, want.bfloat16())
