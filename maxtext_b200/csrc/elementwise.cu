@@ -141,9 +141,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
 // dx = rstd * (g - xhat * mean(g * xhat)) [+ dres], g = dy * (scale + offset);  dscale += sum_rows dy * xhat. `dres` is what reaches the same row past
 // the norm (the residual stream's own gradient): added here, it costs no pass of its own. It joins the norm's gradient as that is stored (bf16), so the sum
 // is the same bits as of a norm and an add on their own.
-// Blocks stride over rows and keep per-column dscale partials in registers; the warps of a block that work on rows of their own
-// (TPR 32) add theirs up in shared memory, each block writes one row into `partial`, and rms_dscale_reduce_kernel adds the rows up
-// in a fixed order: no atomics, so the result is bitwise reproducible.
+// Blocks stride over rows and keep per-column dscale partials in registers; each (block, row slot) writes its partial row into `partial`, and
+// rms_dscale_reduce_kernel adds the rows up in a fixed order: no atomics, so the result is bitwise reproducible.
 // As in the forward pass the next row is fetched before the present one is summed: 110 us for 16384 x 4096 with a stream gradient (537 MB), 192 us without.
 template <int TPR, int VPT>
 __global__ void __launch_bounds__(256, TPR == 32 ? (VPT == 1 ? 4 : 1) : VPT == 1 ? 3 : VPT == 2 ? 2 : 1) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -234,24 +233,8 @@ __global__ void __launch_bounds__(256, TPR == 32 ? (VPT == 1 ? 4 : 1) : VPT == 1
       }
     }
   }
-  if (partial && TPR == 32) {
-    __shared__ float warps[TPR == 32 ? 8 * 512 : 1];     // launched with D <= 512 and 8 warps
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int col = (i * TPR + tid) * 8;
-      if (col < D) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) warps[r_in_block * D + col + e] = ds[i][e];
-      }
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < D; c += blockDim.x) {
-      float a = 0.f;
-      for (int w = 0; w < rows_per_block; ++w) a += warps[w * D + c];
-      partial[(long)blockIdx.x * D + c] = a;
-    }
-  } else if (partial) {
-    float* prow = partial + (long)blockIdx.x * D;
+  if (partial) {
+    float* prow = partial + ((long)blockIdx.x * rows_per_block + r_in_block) * D;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int col = (i * TPR + tid) * 8;
@@ -263,27 +246,46 @@ __global__ void __launch_bounds__(256, TPR == 32 ? (VPT == 1 ? 4 : 1) : VPT == 1
   }
 }
 
-// dscale[c] += sum over partial rows, in a fixed order: 32 row lanes per column, then the lanes one after the other. A thread per
-// column (16 - 32 blocks at the usual widths, one serial chain over all rows) took 47 us for 592 rows of 4096 columns and 95 us for
-// the 4736 rows of a 128-wide head norm; the chain is what bounds it, so the rows are split and the loads of one lane overlap.
-constexpr int kDsLanes = 32;
-__global__ void __launch_bounds__(32 * kDsLanes) rms_dscale_reduce_kernel(const float* __restrict__ partial, int nrows, int D, float* __restrict__ dscale) {
-  __shared__ float lanes[kDsLanes][33];
-  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + x;
-  float a = 0.f;
-  if (c < D) {
-#pragma unroll 8
-    for (int r = y; r < nrows; r += kDsLanes) a += partial[(long)r * D + c];
-  }
-  lanes[y][x] = a;
-  __syncthreads();
-  if (y == 0 && c < D) {
-    a = 0.f;
+// dscale[c] += sum over partial rows, in a fixed order: row r joins sum r % 4 (the last, incomplete four rows all join sum 0), and the four sums meet in
+// pairs. The four serial chains per column are what bounds it, so nothing else may wait in them: a block of 256 threads fetches 16 KB of its COLS columns ahead,
+// and a thread per column and sum adds up the rows that wait in shared memory. Narrow widths have more blocks with eight columns (32-byte pieces); from 1024
+// columns on there are enough with 32. A thread per column that loads what it adds (16 - 32 blocks at the usual widths) took 47 us for 592 rows of 4096
+// columns and 95 us for the 4736 rows of a 128-wide head norm; the whole backward pass takes 60 and 22 us at these sizes now (8192 x 4096, 4800 x 128).
+template <int COLS>
+__global__ void __launch_bounds__(256) rms_dscale_reduce_kernel(const float* __restrict__ partial, int nrows, int D, float* __restrict__ dscale) {
+  constexpr int ROWS = 4096 / COLS, V = COLS / 4, STEP = 256 / V, PER = ROWS / STEP;      // V 16-byte pieces per row, PER of a thread per tile
+  __shared__ __align__(16) float tile[2][ROWS][COLS];
+  __shared__ float sums[4][COLS];
+  const int c0 = blockIdx.x * COLS, piece = (threadIdx.x % V) * 4, r0 = threadIdx.x / V;
+  const int c = threadIdx.x % COLS, j = threadIdx.x / COLS;                                 // column and sum of a thread below 4 COLS
+  const int whole = nrows / 4 * 4;
+  float4 next[PER];
+  auto fetch = [&](int top) {
 #pragma unroll
-    for (int i = 0; i < kDsLanes; ++i) a += lanes[i][x];
-    dscale[c] += a;
+    for (int k = 0; k < PER; ++k) {
+      const int r = top + r0 + k * STEP;
+      if (r < nrows) next[k] = *reinterpret_cast<const float4*>(partial + (long)r * D + c0 + piece);
+    }
+  };
+  fetch(0);
+  float a = 0.f;
+  int buf = 0;
+  for (int top = 0; top < nrows; top += ROWS, buf ^= 1) {
+#pragma unroll
+    for (int k = 0; k < PER; ++k) *reinterpret_cast<float4*>(&tile[buf][r0 + k * STEP][piece]) = next[k];
+    fetch(top + ROWS);
+    __syncthreads();                                         // two buffers in turn: one barrier per tile is enough
+    if (j < 4) {
+      const int n = (whole - top < ROWS ? whole - top : ROWS) / 4;
+#pragma unroll 32
+      for (int i = 0; i < n; ++i) a += tile[buf][4 * i + j][c];
+      if (j == 0 && nrows - top <= ROWS)
+        for (int r = whole - top; r < nrows - top; ++r) a += tile[buf][r][c];
+    }
   }
+  if (j < 4) sums[j][c] = a;
+  __syncthreads();
+  if (j == 0) dscale[c0 + c] += (sums[0][c] + sums[1][c]) + (sums[2][c] + sums[3][c]);
 }
 
 // ------------------------------------------------------------------------------------------------ rotary embedding
@@ -686,17 +688,20 @@ static void launch_rms_bwd(const void* dy, const void* x, const void* scale, con
                                                                   (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, part, rows, D)
   if (vpt <= 1) L(1); else if (vpt <= 2) L(2); else if (vpt <= 4) L(4); else L(8);
 #undef L
-  if (part) rms_dscale_reduce_kernel<<<(D + 31) / 32, 32 * kDsLanes, 0, st>>>(part, grid, D, dscale);
+  if (!part) return;
+  const int prows = grid * (threads / TPR);
+  if (D >= 1024 && D % 32 == 0) rms_dscale_reduce_kernel<32><<<D / 32, 256, 0, st>>>(part, prows, D, dscale);
+  else rms_dscale_reduce_kernel<8><<<D / 8, 256, 0, st>>>(part, prows, D, dscale);
 }
 
 // number of fp32 rows of length D that `partial` must hold for mt_rmsnorm_bwd with a scale gradient
 extern "C" int mt_rmsnorm_bwd_partial_rows(int rows, int D, int sms) {
   const int tpr = D <= 512 ? 32 : 256;
-  return rms_bwd_grid(rows, tpr, sms);
+  return rms_bwd_grid(rows, tpr, sms) * (256 / tpr);
 }
 
-// `partial`: scratch of mt_rmsnorm_bwd_partial_rows(rows, D, sms) x D floats (needed only when dscale is given); every block writes
-// its row, so the scratch needs no clearing.
+// `partial`: scratch of mt_rmsnorm_bwd_partial_rows(rows, D, sms) x D floats (needed only when dscale is given); rows of a
+// block that saw no input row are written as zeros by the kernel, so the scratch needs no clearing.
 extern "C" int mt_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const float* rstd, float offset, const void* dres,
                               void* dx, float* dscale, float* partial, int rows, int D, int sms, cudaStream_t st) {
   if (D % 8 || D > 8 * 256 * 8 || (dscale && !partial)) return -1;

@@ -322,3 +322,29 @@ def test_norm_gradient_rounds_its_factors_once():
     dot = _fma(g[:, e], xh[:, e], dot)
   want = rstd[:, None] * _fma(-xh, (dot / D)[:, None].expand_as(xh), g)
   assert torch.equal(dx, want.bfloat16())
+
+
+@pytest.mark.parametrize("rows,D", [(3, 8), (7, 40), (31, 512), (4736, 128), (6001, 256), (590, 1032), (1300, 1032), (1777, 4096)])
+def test_norm_scale_gradient_in_its_order(rows, D):
+  """The same bits as the sums in their documented order: every block (row slot) a chain of fused steps over its rows, row r of those partial sums
+  to sum r % 4, the last incomplete four to sum 0, and the four in pairs."""
+  E = _E()
+  x, dy = (torch.randn(rows, D, device="cuda").bfloat16() for _ in range(2))
+  rstd = 0.5 + torch.rand(rows, device="cuda")
+  dx, ds = torch.empty_like(x), torch.full((D,), 3.0, device="cuda")
+  E.rmsnorm_bwd(dy, x, torch.ones(D, device="cuda").bfloat16(), rstd, 0.0, dx, ds)
+  per_block = 8 if D <= 512 else 1
+  blocks = min(-(-rows // per_block), 4 * torch.cuda.get_device_properties(0).multi_processor_count)
+  n = blocks * per_block
+  a, xh = dy.float(), x.float() * rstd[:, None]
+  part = torch.zeros(n, D, device="cuda")
+  for top in range(0, rows, n):
+    m = min(n, rows - top)
+    part[:m] = _fma(a[top: top + m], xh[top: top + m], part[:m])
+  sums = torch.zeros(4, D, device="cuda")
+  whole = n // 4 * 4
+  for r in range(0, whole, 4):
+    sums += part[r: r + 4]
+  for r in range(whole, n):
+    sums[0] += part[r]
+  assert torch.equal(ds, 3.0 + ((sums[0] + sums[1]) + (sums[2] + sums[3])))
