@@ -94,10 +94,41 @@ __device__ __forceinline__ void stage_rows_zero(uint32_t box, int row, int c) {
 // ================================================================================================ delta
 // delta[b,h,s] = sum_d dout[b,s,h,d] * out[b,s,h,d] for contiguous [B,S,H,8 LANES] tensors. Bandwidth-bound: LANES threads share a head with one 16-byte
 // load of each tensor, and a thread takes two heads at a time. A warp per head with 4-byte loads moved 2 TB/s (134 us for 2 x 8192 tokens of 32 heads of
-// 128 lanes, 268 MB); 65 us now.
+// 128 lanes, 268 MB).
+// The order of the sum is fixed: products of neighbouring lanes in pairs; pair t joins pair t + 32 (128 lanes), and the 32 sums that are left meet as in a
+// butterfly over the bits 16, 8, 4, 2, 1 of t. A thread's word holds pairs 4 l to 4 l + 3, so the upper bits of t are those of its lane; with 16 lanes the
+// first two exchanges also share out the four pairs.
+template <int LANES>
+__device__ __forceinline__ float delta_sum(const float (&p)[4], int l) {
+  const unsigned all = 0xffffffffu;
+  float v;
+  if (LANES == 16) {
+    const bool b8 = l & 8, b4 = l & 4;
+    float h[2];                                              // lanes with bit 8 keep pairs 2 and 3
+#pragma unroll
+    for (int e = 0; e < 2; ++e) h[e] = (b8 ? p[2 + e] : p[e]) + __shfl_xor_sync(all, b8 ? p[e] : p[2 + e], 8);
+    v = (b4 ? h[1] : h[0]) + __shfl_xor_sync(all, b4 ? h[0] : h[1], 4);      // pair 2 b8 + b4
+    v += __shfl_xor_sync(all, v, 2);
+    v += __shfl_xor_sync(all, v, 1);
+    v += __shfl_xor_sync(all, v, 8);
+    v += __shfl_xor_sync(all, v, 4);
+  } else {
+    float h[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      h[e] = p[e] + __shfl_xor_sync(all, p[e], 4);
+      h[e] += __shfl_xor_sync(all, h[e], 2);
+      h[e] += __shfl_xor_sync(all, h[e], 1);
+    }
+    v = (h[0] + h[2]) + (h[1] + h[3]);
+  }
+  return v;
+}
+
 template <int LANES>
 __global__ void __launch_bounds__(256) delta_kernel(const uint4* __restrict__ dout, const uint4* __restrict__ out, float* __restrict__ delta, int B, int S,
                                                     int H) {
+  static_assert(LANES == 8 || LANES == 16, "heads of 64 or 128 lanes");
   constexpr int HEADS = 256 / LANES;
   const int lane = threadIdx.x % LANES;
   const long n = (long)B * S * H, first = (long)blockIdx.x * 2 * HEADS + threadIdx.x / LANES;
@@ -111,14 +142,13 @@ __global__ void __launch_bounds__(256) delta_kernel(const uint4* __restrict__ do
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162*>(&x[k]), *q = reinterpret_cast<const __nv_bfloat162*>(&y[k]);
-    float acc = 0.f;
+    float pairs[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 f = __bfloat1622float2(p[e]), g = __bfloat1622float2(q[e]);
-      acc += f.x * g.x + f.y * g.y;
+      pairs[e] = __fmaf_rn(f.x, g.x, __fmul_rn(f.y, g.y));
     }
-#pragma unroll
-    for (int off = LANES / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    const float acc = delta_sum<LANES>(pairs, lane);
     const long w = first + k * HEADS;
     if (lane == 0 && w < n) {
       const long bs = w / H;

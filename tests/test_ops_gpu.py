@@ -348,3 +348,33 @@ def test_norm_scale_gradient_in_its_order(rows, D):
   for r in range(whole, n):
     sums[0] += part[r]
   assert torch.equal(ds, 3.0 + ((sums[0] + sums[1]) + (sums[2] + sums[3])))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_row_sums_of_the_gradient_in_their_order(D):
+  """sum_d dout * out, read back through dq: with every probability 1 and no value gradient, dq = -sum * k, and one key is a unit vector. The products are
+  powers of two that do not all fit into fp32 together, so another order of the sum gives other bits."""
+  E = _E()
+  B, S, H = 2, 128, 4
+  g = torch.Generator(device="cuda").manual_seed(D)
+  dout = torch.exp2(torch.randint(-3, 27, (B, S, H, D), device="cuda", generator=g).float()) * (1 - 2 * torch.randint(0, 2, (B, S, H, D), device="cuda", generator=g))
+  out = torch.exp2(torch.randint(-2, 3, (B, S, H, D), device="cuda", generator=g).float())
+  # the large products cancel: every pair of lanes t, t + D / 2 holds opposite ones but for a small rest
+  dout[..., D // 2:] = -dout[..., : D // 2]
+  out[..., D // 2:] = out[..., : D // 2]
+  dout[..., ::7] += 2.0
+  dout, out = dout.bfloat16(), out.bfloat16()
+  q, k, v = torch.zeros(B, S, H, D, device="cuda").bfloat16(), torch.zeros(B, S, H, D, device="cuda").bfloat16(), torch.zeros(B, S, H, D, device="cuda").bfloat16()
+  k[:, 0, :, 0] = 1.0
+  lse = torch.zeros(B, H, S, device="cuda")
+  dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+  E.flash_bwd(dout, q, k, v, out, lse, dq, dk, dv, None, None, None, None, 1.0, 0.0, True, 0, 0, 0)
+  p = dout.float() * out.float()                                  # exact
+  t = p[..., 0::2] + p[..., 1::2]                                 # a pair of neighbouring lanes: one rounding
+  if D == 128:
+    t = t[..., :32] + t[..., 32:]
+  n = 32
+  while n > 1:
+    n //= 2
+    t = t[..., :n] + t[..., n: 2 * n]
+  assert torch.equal(dq[..., 0], (-t[..., 0]).bfloat16())
