@@ -25,15 +25,11 @@ __device__ __forceinline__ float warp_sum2(float v) {
 // and the target logit. Pass 2 (optional): overwrite the row with
 //   dlogits = w * ((1 + 2 z lse) * softmax - onehot(target))
 // so the caller can feed it straight into the dX / dW GEMMs. loss = lse - logit[target] + z * lse^2.
-// Rows are read from HBM once (the second pass finds them in L2) and written once, but with expf the arithmetic took longer than the bytes: 110 us for
-// 2048 x 32000 logits (262 MB, 41 us at copy rate). Exponentials are one ex2 of (f - max) log2(e) each: the difference of two bf16 numbers is exact or has the
-// rounding it had before, and one more rounding of its product leaves terms that matter to the sum (|f - max| < 8) within 5e-7, as expf does, and a thread has four vectors in flight. 61 us now.
-constexpr float kLog2e = 1.4426950408889634f;
-__device__ __forceinline__ float exp_of(float x) {          // e^x for x <= 0 up to rounding; e^-inf = 0
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * kLog2e));
-  return y;
-}
+// Rows are read from HBM once (the second pass finds them in L2) and written once. A row is 1024 chains of vectors (chain c: vectors c, c + 1024, ...), each
+// with a maximum and a sum of its own, whose results meet warp by warp: that fixes the order of the sums. A thread works on CHAINS of them, so that it has four
+// vectors in flight and that a block can be as small as its row allows. Bytes (41 us at copy rate for 2048 x 32000) and the exponentials of both passes bound it:
+// 72 us for 2048 x 32000, 220 us for 2048 x 102400; 88 and 240 us with one chain of one vector at a time. Exponentials are expf in full: the loss and the
+// gradient are fp32 results.
 __device__ __forceinline__ void unpack(const bf16x8& p, float (&f)[8]) {
   const uint32_t w[4] = {p.q.x, p.q.y, p.q.z, p.q.w};
 #pragma unroll
@@ -43,60 +39,60 @@ __device__ __forceinline__ void unpack(const bf16x8& p, float (&f)[8]) {
   }
 }
 
-__global__ void __launch_bounds__(1024) xent_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__ targets,
-                                                    const float* __restrict__ weights, float z_loss, float* __restrict__ loss_out,
-                                                    float* __restrict__ z_out, long ld, int V, int write_grad) {
+template <int CHAINS>
+__global__ void __launch_bounds__(1024 / CHAINS) xent_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__ targets,
+                                                             const float* __restrict__ weights, float z_loss, float* __restrict__ loss_out,
+                                                             float* __restrict__ z_out, long ld, int V, int write_grad) {
   __shared__ float s_m[32], s_s[32];
   __shared__ float s_lse;
+  constexpr int T = 1024 / CHAINS;
   const long row = blockIdx.x;
   __nv_bfloat16* lrow = logits + row * ld;
   const int tgt = targets[row];
   const int nvec = V / 8;
-  float m = -INFINITY, s = 0.f;
-  constexpr int U = 4;                                       // vectors of a thread in flight; a missing one counts as -inf
-  for (int i = threadIdx.x; i < nvec; i += U * blockDim.x) {
-    bf16x8 p[U];
+  float m[CHAINS], s[CHAINS];
 #pragma unroll
-    for (int k = 0; k < U; ++k) {
-      p[k].q = make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);
-      if (i + k * (int)blockDim.x < nvec) p[k] = *reinterpret_cast<const bf16x8*>(lrow + (i + k * blockDim.x) * 8);
+  for (int c = 0; c < CHAINS; ++c) { m[c] = -INFINITY; s[c] = 0.f; }
+  for (int i = threadIdx.x; i < nvec; i += 4 * T) {          // four vectors: 4 / CHAINS of each chain, in order
+    bf16x8 p[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * T < nvec) p[k] = *reinterpret_cast<const bf16x8*>(lrow + (i + k * T) * 8);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k * T < nvec) {
+        const int c = k % CHAINS;
+        float f[8];
+        unpack(p[k], f);
+        float nm = m[c];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) nm = fmaxf(nm, f[e]);
+        const float base = nm == -INFINITY ? 0.f : nm;       // nothing but -inf so far: every term is 0
+        float acc = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc += expf(f[e] - base);
+        s[c] = s[c] * expf(m[c] - base) + acc;
+        m[c] = nm;
+      }
     }
-    float nm = m;
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      float f[8];
-      unpack(p[k], f);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) nm = fmaxf(nm, f[e]);
-    }
-    const float base = nm == -INFINITY ? 0.f : nm;           // nothing but -inf so far: every term is 0
-    s *= exp_of(m - base);
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      float f[8], acc = 0.f;
-      unpack(p[k], f);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc += exp_of(f[e] - base);
-      s += acc;
-    }
-    m = nm;
   }
-  for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) {   // tail when V % 8 != 0
+  for (int i = nvec * 8 + threadIdx.x; i < V; i += T) {      // tail when V % 8 != 0: at most 7 logits
     const float f = __bfloat162float(lrow[i]);
-    const float nm = fmaxf(m, f), base = nm == -INFINITY ? 0.f : nm;
-    s = s * expf(m - base) + expf(f - base);
-    m = nm;
+    const float nm = fmaxf(m[0], f), base = nm == -INFINITY ? 0.f : nm;
+    s[0] = s[0] * expf(m[0] - base) + expf(f - base);
+    m[0] = nm;
   }
   // block reduce (max, sum)
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  float wm = warp_max(m);
-  float ws = warp_sum2(s * ((m == -INFINITY) ? 0.f : expf(m - wm)));
-  if (l == 0) { s_m[w] = wm; s_s[w] = ws; }
+#pragma unroll
+  for (int c = 0; c < CHAINS; ++c) {
+    const float wm = warp_max(m[c]);
+    const float ws = warp_sum2(s[c] * ((m[c] == -INFINITY) ? 0.f : expf(m[c] - wm)));
+    if (l == 0) { s_m[w + c * (T / 32)] = wm; s_s[w + c * (T / 32)] = ws; }
+  }
   __syncthreads();
   if (w == 0) {
-    const int nw = blockDim.x >> 5;
-    float mm = (l < nw) ? s_m[l] : -INFINITY;
-    float ss = (l < nw) ? s_s[l] : 0.f;
+    const float mm = s_m[l], ss = s_s[l];
     const float gm = warp_max(mm);
     const float gs = warp_sum2(ss * ((mm == -INFINITY) ? 0.f : expf(mm - gm)));
     if (l == 0) {
@@ -114,12 +110,12 @@ __global__ void __launch_bounds__(1024) xent_kernel(__nv_bfloat16* __restrict__ 
   const float wgt = weights ? weights[row] : 1.f;
   const float coef = wgt * (1.f + 2.f * z_loss * lse);
 #pragma unroll 4
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+  for (int i = threadIdx.x; i < nvec; i += T) {
     const bf16x8 p = *reinterpret_cast<const bf16x8*>(lrow + i * 8);
     float f[8];
     unpack(p, f);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] = coef * exp_of(f[e] - lse);
+    for (int e = 0; e < 8; ++e) f[e] = coef * expf(f[e] - lse);
     if (tgt >> 3 == i) {
 #pragma unroll
       for (int e = 0; e < 8; ++e)
@@ -133,7 +129,7 @@ __global__ void __launch_bounds__(1024) xent_kernel(__nv_bfloat16* __restrict__ 
     }
     *reinterpret_cast<uint4*>(lrow + i * 8) = make_uint4(w[0], w[1], w[2], w[3]);
   }
-  for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) {
+  for (int i = nvec * 8 + threadIdx.x; i < V; i += T) {
     float a = coef * expf(__bfloat162float(lrow[i]) - lse);
     if (i == tgt) a -= wgt;
     lrow[i] = __float2bfloat16_rn(a);
@@ -236,10 +232,14 @@ extern "C" int mt_xent(void* logits, const int* targets, const float* weights, f
                        long ld, int V, int write_grad, cudaStream_t st) {
   if (rows <= 0) return 0;
   if (ld % 8) return -1;
-  // smaller blocks overlap their phases better, but the rows of the resident ones must be found in L2 again (126 MB) by the second pass: 256, 512 and 1024
-  // threads take 61, 66, 84 us for 2048 x 32000 logits, 244, 185, 203 for 2048 x 102400 and 365, 306, 274 for 1999 x 151936
-  const int threads = V <= 32768 ? 256 : V <= 131072 ? 512 : 1024;
-  xent_kernel<<<(unsigned)rows, threads, 0, st>>>((__nv_bfloat16*)logits, targets, weights, z_loss, loss_out, z_out, ld, V, write_grad);
+  // smaller blocks overlap their phases better, but the rows of the resident ones must be found in L2 again (126 MB) by the second pass.
+  // 256, 512 and 1024 threads, us: 2048 x 32000 72, 80, 100; x 49152 108, 115, 137; x 65536 152, 145, 166; x 131072 315, 289, 296; 1999 x 151936 368, 350, 344
+  auto run = [&](auto kernel, int threads) {
+    kernel<<<(unsigned)rows, threads, 0, st>>>((__nv_bfloat16*)logits, targets, weights, z_loss, loss_out, z_out, ld, V, write_grad);
+  };
+  if (V <= 49152) run(xent_kernel<4>, 256);
+  else if (V <= 131072) run(xent_kernel<2>, 512);
+  else run(xent_kernel<1>, 1024);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

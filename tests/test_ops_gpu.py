@@ -378,3 +378,62 @@ def test_row_sums_of_the_gradient_in_their_order(D):
     n //= 2
     t = t[..., :n] + t[..., n: 2 * n]
   assert torch.equal(dq[..., 0], (-t[..., 0]).bfloat16())
+
+
+def _butterfly(v, op):
+  """What a warp's exchanges over 16, 8, 4, 2, 1 lanes leave of v [..., 32]."""
+  n = 32
+  while n > 1:
+    n //= 2
+    v = op(v[..., :n], v[..., n: 2 * n])
+  return v[..., 0]
+
+
+@pytest.mark.parametrize("V", [8, 100, 8191, 32000, 32003, 102400, 151936])
+def test_cross_entropy_in_its_order_and_with_full_exponentials(V):
+  """Loss and gradient are the same bits as 1024 chains of eight logits each (chain c: vectors c, c + 1024, ...; the tail on chains 0 to 6), joined warp by
+  warp, with fp32's own exponential. Whole vectors of -inf come before, between and behind finite ones."""
+  E = _E()
+  g = torch.Generator(device="cuda").manual_seed(V)
+  rows, ld, nvec = 7, (V + 7) // 8 * 8, V // 8
+  store = (torch.randn(rows, ld, device="cuda", generator=g) * 6).bfloat16()
+  if nvec > 3:
+    store[1, : (nvec // 2) * 8] = float("-inf")                  # the first vectors of every chain
+    store[2, 8: 8 * (nvec - 1)] = float("-inf")
+    store[3, (nvec - 1) * 8: nvec * 8] = float("-inf")
+  tgt = torch.full((rows,), V - 1, device="cuda", dtype=torch.int32)
+  store[:, V - 1] = 1.0
+  wt = torch.rand(rows, device="cuda", generator=g) + 0.5
+  x, inf = store[:, :V].float(), torch.tensor(float("-inf"), device="cuda")
+  m, s = torch.full((rows, 1024), float("-inf"), device="cuda"), torch.zeros(rows, 1024, device="cuda")
+
+  def step(f, n):
+    """f [rows, n, k]: k more logits of chains 0 .. n - 1."""
+    nm = torch.maximum(m[:, :n], f.amax(-1))
+    base = torch.where(nm == inf, 0.0, nm)
+    acc = torch.zeros_like(nm)
+    for e in range(f.shape[-1]):
+      acc = acc + torch.exp(f[..., e] - base)
+    s[:, :n] = _fma(s[:, :n], torch.exp(m[:, :n] - base), acc)
+    m[:, :n] = nm
+  for top in range(0, nvec, 1024):
+    n = min(1024, nvec - top)
+    step(x[:, top * 8: (top + n) * 8].view(rows, n, 8), n)
+  if V % 8:
+    step(x[:, nvec * 8:, None], V % 8)
+  join = lambda m, s: (_butterfly(m, torch.maximum), m, s)  # noqa: E731
+  for _ in range(2):                                              # the 32 lanes of every warp, then the 32 warps
+    m, s = m.view(rows, -1, 32), s.view(rows, -1, 32)
+    top, m, s = join(m, s)
+    s = _butterfly(s * torch.where(m == inf, 0.0, torch.exp(m - top[..., None])), torch.add)
+    m = top
+  lse = (m + torch.log(s)).view(rows)
+  loss, z = torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda")
+  work = store.clone()
+  E.xent_fwd_bwd(work[:, :V], tgt, wt, 0.0, loss, z, True)
+  assert bool(torch.isfinite(loss).all()) and torch.equal(loss, lse - x[:, V - 1])
+  p = wt[:, None] * torch.exp(x - lse[:, None])
+  assert torch.equal(work[:, : V - 1], p[:, : V - 1].bfloat16())
+  last = p[:, V - 1] - wt
+  assert bool(((work[:, V - 1].float() - last).abs() <= 2 ** -8 * last.abs()).all())
+  assert torch.equal(work[:, V:], store[:, V:])
