@@ -384,24 +384,9 @@ __global__ void __launch_bounds__(512) rope_vec_kernel(__nv_bfloat16* __restrict
 }
 
 // ------------------------------------------------------------------------------------------------ gated activation
-// 1 / (1 + e^-g) with the denominator d, which is kept finite: a reciprocal estimate and one Newton step on its residual, without the division's branches
-// (under the power cap of a long training step its instructions took longer than the bytes).
-__device__ __forceinline__ float sigmoid_of(float g, float& d) {
-  d = 1.f + fminf(__expf(-g), 3e38f);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));       // 0 above 2^126, where the true value is below 2e-38
-  return __fmaf_rn(__fmaf_rn(-r, d, 1.f), r, r);
-}
-// g / (1 + e^-g), the quotient corrected by its own residual, so that it rounds like the division
-__device__ __forceinline__ float silu(float g) {
-  float d;
-  const float r = sigmoid_of(g, d), q = g * r;
-  return g > 80.f ? g : __fmaf_rn(__fmaf_rn(-q, d, g), r, q);  // there d is 1
-}
-
 __device__ __forceinline__ float act_apply(float g, int code) {
   switch (code) {
-    case 0: return silu(g);
+    case 0: return g / (1.f + __expf(-g));                                                         // silu
     case 1: { const float k = 0.7978845608028654f; return 0.5f * g * (1.f + tanhf(k * (g + 0.044715f * g * g * g))); }  // gelu (tanh)
     case 2: return g > 0.f ? g : 0.f;                                                              // relu
     default: return g;                                                                             // linear
@@ -409,7 +394,7 @@ __device__ __forceinline__ float act_apply(float g, int code) {
 }
 __device__ __forceinline__ float act_grad(float g, int code) {
   switch (code) {
-    case 0: { float d; const float s = sigmoid_of(g, d); return s * (1.f + g * (1.f - s)); }
+    case 0: { const float s = 1.f / (1.f + __expf(-g)); return s * (1.f + g * (1.f - s)); }
     case 1: {
       const float k = 0.7978845608028654f;
       const float u = k * (g + 0.044715f * g * g * g);

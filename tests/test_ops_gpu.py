@@ -437,3 +437,26 @@ def test_cross_entropy_in_its_order_and_with_full_exponentials(V):
   last = p[:, V - 1] - wt
   assert bool(((work[:, V - 1].float() - last).abs() <= 2 ** -8 * last.abs()).all())
   assert torch.equal(work[:, V:], store[:, V:])
+
+
+def test_gated_silu_over_every_gate():
+  """Every bf16 gate with up and dy = 1, against fp64. __expf is within 2 + 1.173 |g| ulps (|g| < 90: 108 * 2**-23 < 2**-16), two more roundings and the one
+  to bf16. Results down to bf16's smallest normal number are kept; where e^-g overflows (g < -88.73) the quotient is -0, as at -inf / inf a NaN."""
+  E = _E()
+  gate = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+  gu = torch.cat([gate, torch.ones_like(gate)])[None].contiguous()
+  out, dgu = torch.empty(1, 65536, device="cuda", dtype=torch.bfloat16), torch.empty_like(gu)
+  E.gated_act_fwd(gu, out, 0)
+  E.gated_act_bwd(torch.ones_like(out), gu, dgu, 0)
+  g = gate.double()
+  sig = torch.sigmoid(g)
+  want, grad = g * sig, sig * (1 + g * (1 - sig))
+  tiny, rel = 2.0 ** -126, 2.0 ** -8
+  ok = torch.isfinite(g) & (g > -88.7)
+  for got in (out[0], dgu[0, 65536:]):                            # the activation, and the gradient of `up`
+    assert bool(((got.double() - want).abs() <= rel * want.abs() + tiny)[ok].all())
+    assert bool((got[(g <= -88.75) & torch.isfinite(g)] == 0).all())
+    assert bool(torch.isnan(got[torch.isnan(g) | (g == float("-inf"))]).all()) and bool((got[g == float("inf")] == float("inf")).all())
+  # s * (1 + g * (1 - s)) cancels around its zero at g = -1.28: four fp32 roundings of terms below 2 and the exponential's error in both of its uses
+  err = (dgu[0, :65536].double() - grad).abs()
+  assert bool((err <= rel * grad.abs() + sig * (1 + g.abs()) * 2.0 ** -15 + tiny)[ok].all())
