@@ -216,14 +216,32 @@ int64_t kernel_status(bool reset) {
   return v;
 }
 
+// The kernels below move 16 bytes at a time. A tensor that starts elsewhere (a slice of a flat buffer) takes part through a copy that does not.
+bool on16(const torch::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+torch::Tensor in16(const torch::Tensor& t) { return on16(t) ? t : t.clone(); }
+c10::optional<torch::Tensor> in16(const c10::optional<torch::Tensor>& t) { return t ? c10::optional<torch::Tensor>(in16(*t)) : t; }
+struct Out16 {
+  torch::Tensor user, t;
+  explicit Out16(const torch::Tensor& u) : user(u), t(on16(u) ? u : torch::empty_like(u)) {}
+  void* ptr() const { return t.data_ptr(); }
+  void done() { if (!t.is_same(user)) user.copy_(t); }
+};
+
 void rmsnorm_fwd(const torch::Tensor& x, const c10::optional<torch::Tensor>& scale, double eps, double offset, torch::Tensor& y,
                  const c10::optional<torch::Tensor>& rstd, const c10::optional<torch::Tensor>& add, const c10::optional<torch::Tensor>& sum) {
   TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && x.dim() == 2 && bool(add) == bool(sum));
   for (const auto& t : {add, sum}) TORCH_CHECK(!t || (t->is_contiguous() && t->numel() == x.numel() && t->scalar_type() == x.scalar_type()));
   c10::cuda::CUDAGuard guard(x.device());
-  check(mt_rmsnorm_fwd(x.data_ptr(), add ? add->data_ptr() : nullptr, sum ? sum->data_ptr() : nullptr, scale ? scale->data_ptr() : nullptr, (float)eps, (float)offset, y.data_ptr(),
-                       rstd ? rstd->data_ptr<float>() : nullptr, (int)x.size(0), (int)x.size(1), cur_stream()),
+  const torch::Tensor xa = in16(x);
+  const auto sa = in16(scale), aa = in16(add);
+  Out16 ya(y);
+  c10::optional<Out16> so;
+  if (sum) so.emplace(*sum);
+  check(mt_rmsnorm_fwd(xa.data_ptr(), aa ? aa->data_ptr() : nullptr, so ? so->ptr() : nullptr, sa ? sa->data_ptr() : nullptr, (float)eps, (float)offset,
+                       ya.ptr(), rstd ? rstd->data_ptr<float>() : nullptr, (int)x.size(0), (int)x.size(1), cur_stream()),
         "mt_rmsnorm_fwd");
+  ya.done();
+  if (so) so->done();
 }
 
 void rmsnorm_bwd(const torch::Tensor& dy, const torch::Tensor& x, const c10::optional<torch::Tensor>& scale, const torch::Tensor& rstd,
@@ -234,10 +252,14 @@ void rmsnorm_bwd(const torch::Tensor& dy, const torch::Tensor& x, const c10::opt
   torch::Tensor partial;
   if (dscale) partial = torch::empty({mt_rmsnorm_bwd_partial_rows((int)x.size(0), (int)x.size(1), num_sms()), x.size(1)},
                                      torch::TensorOptions().dtype(torch::kFloat32).device(x.device()));
-  check(mt_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), scale ? scale->data_ptr() : nullptr, rstd.data_ptr<float>(), (float)offset,
-                       dres ? dres->data_ptr() : nullptr, dx.data_ptr(), dscale ? dscale->data_ptr<float>() : nullptr, dscale ? partial.data_ptr<float>() : nullptr,
-                       (int)x.size(0), (int)x.size(1), num_sms(), cur_stream()),
+  const torch::Tensor da = in16(dy), xa = in16(x);
+  const auto sa = in16(scale), ra = in16(dres);
+  Out16 dxa(dx);
+  check(mt_rmsnorm_bwd(da.data_ptr(), xa.data_ptr(), sa ? sa->data_ptr() : nullptr, rstd.data_ptr<float>(), (float)offset, ra ? ra->data_ptr() : nullptr,
+                       dxa.ptr(), dscale ? dscale->data_ptr<float>() : nullptr, dscale ? partial.data_ptr<float>() : nullptr, (int)x.size(0),
+                       (int)x.size(1), num_sms(), cur_stream()),
         "mt_rmsnorm_bwd");
+  dxa.done();
 }
 
 void rope_inplace(torch::Tensor& x, const torch::Tensor& pos, const torch::Tensor& inv_ts, int64_t n_rot, bool interleaved, bool inverse,
@@ -253,14 +275,19 @@ void rope_inplace(torch::Tensor& x, const torch::Tensor& pos, const torch::Tenso
 void gated_act_fwd(const torch::Tensor& gu, torch::Tensor& out, int64_t code) {
   TORCH_CHECK(gu.is_contiguous() && out.is_contiguous() && gu.size(1) == 2 * out.size(1));
   c10::cuda::CUDAGuard guard(gu.device());
-  check(mt_gated_act_fwd(gu.data_ptr(), out.data_ptr(), gu.size(0), (int)out.size(1), (int)code, cur_stream()), "gated_act_fwd");
+  const torch::Tensor ga = in16(gu);
+  Out16 oa(out);
+  check(mt_gated_act_fwd(ga.data_ptr(), oa.ptr(), gu.size(0), (int)out.size(1), (int)code, cur_stream()), "gated_act_fwd");
+  oa.done();
 }
 
 void gated_act_bwd(const torch::Tensor& dy, const torch::Tensor& gu, torch::Tensor& dgu, int64_t code) {
   TORCH_CHECK(gu.is_contiguous() && dy.is_contiguous() && dgu.is_contiguous());
   c10::cuda::CUDAGuard guard(gu.device());
-  check(mt_gated_act_bwd(dy.data_ptr(), gu.data_ptr(), dgu.data_ptr(), gu.size(0), (int)dy.size(1), (int)code, cur_stream()),
-        "gated_act_bwd");
+  const torch::Tensor da = in16(dy), ga = in16(gu);
+  Out16 oa(dgu);
+  check(mt_gated_act_bwd(da.data_ptr(), ga.data_ptr(), oa.ptr(), gu.size(0), (int)dy.size(1), (int)code, cur_stream()), "gated_act_bwd");
+  oa.done();
 }
 
 // forward: (q [N, H, nope + rope], kr [N, rope] rows of any stride, kv [N, H, nope + vd]) -> (qo, k [N, H, nope + rope], v [N, H, vd])
@@ -309,9 +336,15 @@ void xent_fwd_bwd(torch::Tensor& logits, const torch::Tensor& targets, const tor
   TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1 && logits.scalar_type() == torch::kBFloat16);
   TORCH_CHECK(targets.scalar_type() == torch::kInt32 && weights.scalar_type() == torch::kFloat32);
   c10::cuda::CUDAGuard guard(logits.device());
-  check(mt_xent(logits.data_ptr(), targets.data_ptr<int>(), weights.data_ptr<float>(), (float)z_loss, loss.data_ptr<float>(),
-                z.data_ptr<float>(), logits.size(0), logits.stride(0), (int)logits.size(1), write_grad, cur_stream()),
+  torch::Tensor rows = logits;
+  if (!on16(logits) && logits.stride(0) % 8 == 0) {          // rows are refused where their stride is no multiple of 8
+    rows = torch::empty({logits.size(0), (logits.size(1) + 7) / 8 * 8}, logits.options()).narrow(1, 0, logits.size(1));
+    rows.copy_(logits);
+  }
+  check(mt_xent(rows.data_ptr(), targets.data_ptr<int>(), weights.data_ptr<float>(), (float)z_loss, loss.data_ptr<float>(),
+                z.data_ptr<float>(), rows.size(0), rows.stride(0), (int)rows.size(1), write_grad, cur_stream()),
         "mt_xent");
+  if (write_grad && !rows.is_same(logits)) logits.copy_(rows);
 }
 
 void adamw(torch::Tensor& p, const torch::Tensor& g, torch::Tensor& m, torch::Tensor& v, const c10::optional<torch::Tensor>& shadow,

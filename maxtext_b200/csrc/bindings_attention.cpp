@@ -85,11 +85,13 @@ void flash_bwd(const torch::Tensor& dout, const torch::Tensor& q, const torch::T
   TORCH_CHECK(bool(seg_q) == bool(seg_k) && bool(pos_q) == bool(pos_k), "segment ids / positions must be given for queries and keys together");
   const int B = (int)q.size(0), Sq = (int)q.size(1), Skv = (int)k.size(1), Hq = (int)q.size(2);
   TORCH_CHECK(lse.numel() == (int64_t)B * Hq * Sq && out.size(0) == B && out.size(1) == Sq && out.size(2) == Hq && out.size(3) == v.size(3));
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(dout.data_ptr()) % 16 == 0, "flash_bwd: dout starts off a 16-byte boundary");      // no tensor map for it
   c10::cuda::CUDAGuard guard(q.device());
+  const torch::Tensor oa = reinterpret_cast<uintptr_t>(out.data_ptr()) % 16 == 0 ? out : out.clone();       // its row sums take 16 bytes at a time
   auto delta = torch::empty({B, Hq, Sq}, lse.options());
   torch::Tensor tiles;
   if (pos_q) tiles = torch::empty({mt_attn_tile_ints(B, Sq, Skv)}, torch::dtype(torch::kInt32).device(q.device()));
-  int rc = mt_flash_bwd(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr<float>(), delta.data_ptr<float>(),
+  int rc = mt_flash_bwd(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), oa.data_ptr(), lse.data_ptr<float>(), delta.data_ptr<float>(),
                         dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), opt_int(seg_q, (int64_t)B * Sq, "seg_q"), opt_int(seg_k, (int64_t)B * Skv, "seg_k"),
                         opt_int(pos_q, (int64_t)B * Sq, "pos_q"), opt_int(pos_k, (int64_t)B * Skv, "pos_k"), pos_q ? tiles.data_ptr<int>() : nullptr,
                         B, Sq, Skv, Hq, (int)k.size(2), (int)q.size(3), (int)v.size(3), q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1), v.stride(0),

@@ -849,7 +849,8 @@ class _LatentHeadsFn(torch.autograd.Function):
     N, H, _ = dqo.shape
     dq, dkr = torch.empty_like(dqo, memory_format=torch.contiguous_format), torch.empty(N, rope_d, dtype=dqo.dtype, device=dqo.device)
     dkv = torch.empty(N, H, kvw, dtype=dqo.dtype, device=dqo.device)
-    backend.ext().latent_heads(True, dqo.contiguous(), dk.contiguous(), dv.contiguous(), dq, dkr, dkv, pos, inv_ts, nope, scale, interleaved)
+    whole = lambda t: t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)  # noqa: E731
+    backend.ext().latent_heads(True, whole(dqo), whole(dk), whole(dv), dq, dkr, dkv, pos, inv_ts, nope, scale, interleaved)
     return dq, dkr, dkv, None, None, None, None, None
 
 

@@ -460,3 +460,57 @@ def test_gated_silu_over_every_gate():
   # s * (1 + g * (1 - s)) cancels around its zero at g = -1.28: four fp32 roundings of terms below 2 and the exponential's error in both of its uses
   err = (dgu[0, :65536].double() - grad).abs()
   assert bool((err <= rel * grad.abs() + sig * (1 + g.abs()) * 2.0 ** -15 + tiny)[ok].all())
+
+
+@pytest.mark.parametrize("at", [1, 2, 4])
+def test_views_that_start_off_a_16_byte_boundary(at):
+  """Contiguous slices of a flat buffer, `at` elements in: the same bits as of tensors that start on a boundary, and nothing around them is written."""
+  E = _E()
+  around = []
+
+  def off(t):
+    flat = torch.full((t.numel() + 16,), 7.0, device="cuda", dtype=t.dtype)
+    around.append((flat, t.numel()))
+    v = flat[at: at + t.numel()].view(t.shape)
+    return v.copy_(t)
+  rows, D, F = 37, 264, 520
+  x, a, dy, dres = (torch.randn(rows, D, device="cuda").bfloat16() for _ in range(4))
+  scale, rstd = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16(), torch.empty(rows, device="cuda")
+  gu, dh = torch.randn(rows, 2 * F, device="cuda").bfloat16(), torch.randn(rows, F, device="cuda").bfloat16()
+  logits = torch.randn(rows, 104, device="cuda").bfloat16()
+  tgt, wt = torch.arange(rows, device="cuda", dtype=torch.int32), torch.rand(rows, device="cuda")
+  q, k, v, do = (torch.randn(2, 65, h, 64, device="cuda").bfloat16() for h in (4, 2, 2, 4))
+
+  def run(f):
+    new = lambda t: f(torch.zeros_like(t))  # noqa: E731
+    y, s, dx = new(x), new(x), new(x)
+    E.rmsnorm_fwd(f(x), f(scale), 1e-5, 0.0, y, rstd, f(a), s)
+    ds = torch.zeros(D, device="cuda")
+    E.rmsnorm_bwd(f(dy), f(x), f(scale), rstd, 0.0, dx, ds, f(dres))
+    h, dgu = new(dh), new(gu)
+    E.gated_act_fwd(f(gu), h, 0)
+    E.gated_act_bwd(f(dh), f(gu), dgu, 0)
+    lg, loss, z = f(logits), torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda")
+    E.xent_fwd_bwd(lg[:, :99], tgt, wt, 0.0, loss, z, True)
+    out, lse = torch.zeros_like(q), torch.empty(2, 4, 65, device="cuda")
+    E.flash_fwd(q, k, v, out, lse, None, None, None, None, None, 0.1, 0.0, True, 0, 0, 0)
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    E.flash_bwd(do, q, k, v, f(out), lse, dq, dk, dv, None, None, None, None, 0.1, 0.0, True, 0, 0, 0)
+    return [t.clone() for t in (y, s, dx, ds, h, dgu, lg, loss, z, dq, dk, dv)]
+  want, got = run(lambda t: t.clone()), run(off)
+  for i, (w, g) in enumerate(zip(want, got)):
+    assert torch.equal(w, g), i
+  for flat, n in around:
+    assert bool((flat[:at] == 7).all()) and bool((flat[at + n:] == 7).all())
+  # a gradient of latent attention's heads that comes as such a slice
+  from maxtext_b200.ops import functional as Fn
+  B, S, H, nope, rope, vd = 1, 5, 2, 16, 16, 8
+  inv, pos = ref.rope_inv_timescale(rope, 1, 10000).cuda(), torch.arange(S, device="cuda")[None]
+  src = [torch.randn(*s, device="cuda").bfloat16() for s in ((B, S, H, nope + rope), (B, S, rope), (B, S, H, nope + vd))]
+  up = [torch.randn(B, S, H, n, device="cuda").bfloat16() for n in (nope + rope, nope + rope, vd)]
+  grads = []
+  for f in (lambda t: t, off):
+    leaves = [t.clone().requires_grad_(True) for t in src]
+    grads.append(torch.autograd.grad(Fn.latent_heads(*leaves, pos, inv, nope, 0.3), leaves, [f(t) for t in up]))
+  for w, g in zip(*grads):
+    assert torch.equal(w, g)
