@@ -406,64 +406,64 @@ __device__ __forceinline__ float act_grad(float g, int code) {
   }
 }
 
-// gu [rows, 2F] = [gate | up] -> out [rows, F]. Bandwidth-bound: a block takes 256 neighbouring 16-byte columns of two rows at a time, so that a thread has
-// four (backward: six) loads in flight and no index to divide. One vector per thread out of a flat index with 64-bit divisions, as it was, moved
-// 4.0 TB/s: 354 us forward and 605 us backward for 16384 rows of 14336 lanes, against 255 and 362 us here.
+// gu [rows, 2F] = [gate | up] -> out [rows, F]. Bandwidth-bound: a thread takes a 16-byte column of two rows at a time, so that it has four (backward: six)
+// loads in flight and no index to divide; a block is as wide as the row needs (gated_block) and takes several pairs of rows where that is less than 256
+// threads. One vector per thread out of a flat index with 64-bit divisions took 283 us forward and 482 us backward for 16384 x 14336 and 51 and 80 us for
+// 24576 x 1408; 246, 371, 47 and 70 us here (5.7 TB/s). The division of the sigmoid is what keeps the forward pass from copy rate.
 template <int CODE>
-__global__ void __launch_bounds__(256) gated_act_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long rows, int F) {
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
+__global__ void __launch_bounds__(256) gated_act_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long rows, int F,
+                                                            unsigned across) {
+  const int c = (blockIdx.x % across * blockDim.x + threadIdx.x) * 8;
+  const long r = (blockIdx.x / across * (long)blockDim.y + threadIdx.y) * 2;
   if (c >= F) return;
-  for (long r = blockIdx.y * 2l; r < rows; r += gridDim.y * 2l) {
-    bf16x8 g[2], u[2];
+  bf16x8 g[2], u[2];
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-      if (r + k < rows) {
-        g[k] = *reinterpret_cast<const bf16x8*>(gu + (r + k) * 2 * F + c);
-        u[k] = *reinterpret_cast<const bf16x8*>(gu + (r + k) * 2 * F + F + c);
-      }
+  for (int k = 0; k < 2; ++k)
+    if (r + k < rows) {
+      g[k] = *reinterpret_cast<const bf16x8*>(gu + (r + k) * 2 * F + c);
+      u[k] = *reinterpret_cast<const bf16x8*>(gu + (r + k) * 2 * F + F + c);
+    }
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-      if (r + k < rows) {
-        float a[8], b[8], o[8];
-        unpack8(g[k], a);
-        unpack8(u[k], b);
+  for (int k = 0; k < 2; ++k)
+    if (r + k < rows) {
+      float a[8], b[8], o[8];
+      unpack8(g[k], a);
+      unpack8(u[k], b);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = act_apply(a[e], CODE) * b[e];
-        *reinterpret_cast<bf16x8*>(out + (r + k) * F + c) = pack8(o);
-      }
-  }
+      for (int e = 0; e < 8; ++e) o[e] = act_apply(a[e], CODE) * b[e];
+      *reinterpret_cast<bf16x8*>(out + (r + k) * F + c) = pack8(o);
+    }
 }
 
 template <int CODE>
-__global__ void __launch_bounds__(256) gated_act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gu,
-                                                            __nv_bfloat16* __restrict__ dgu, long rows, int F) {
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
+__global__ void __launch_bounds__(256, 5) gated_act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gu,
+                                                            __nv_bfloat16* __restrict__ dgu, long rows, int F, unsigned across) {
+  const int c = (blockIdx.x % across * blockDim.x + threadIdx.x) * 8;
+  const long r = (blockIdx.x / across * (long)blockDim.y + threadIdx.y) * 2;
   if (c >= F) return;
-  for (long r = blockIdx.y * 2l; r < rows; r += gridDim.y * 2l) {
-    bf16x8 g[2], u[2], d[2];
+  bf16x8 g[2], u[2], d[2];
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-      if (r + k < rows) {
-        g[k] = *reinterpret_cast<const bf16x8*>(gu + (r + k) * 2 * F + c);
-        u[k] = *reinterpret_cast<const bf16x8*>(gu + (r + k) * 2 * F + F + c);
-        d[k] = *reinterpret_cast<const bf16x8*>(dy + (r + k) * F + c);
+  for (int k = 0; k < 2; ++k)
+    if (r + k < rows) {
+      g[k] = *reinterpret_cast<const bf16x8*>(gu + (r + k) * 2 * F + c);
+      u[k] = *reinterpret_cast<const bf16x8*>(gu + (r + k) * 2 * F + F + c);
+      d[k] = *reinterpret_cast<const bf16x8*>(dy + (r + k) * F + c);
+    }
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (r + k < rows) {
+      float a[8], b[8], t[8], dg[8], du[8];
+      unpack8(g[k], a);
+      unpack8(u[k], b);
+      unpack8(d[k], t);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        dg[e] = t[e] * b[e] * act_grad(a[e], CODE);
+        du[e] = t[e] * act_apply(a[e], CODE);
       }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-      if (r + k < rows) {
-        float a[8], b[8], t[8], dg[8], du[8];
-        unpack8(g[k], a);
-        unpack8(u[k], b);
-        unpack8(d[k], t);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          dg[e] = t[e] * b[e] * act_grad(a[e], CODE);
-          du[e] = t[e] * act_apply(a[e], CODE);
-        }
-        *reinterpret_cast<bf16x8*>(dgu + (r + k) * 2 * F + c) = pack8(dg);
-        *reinterpret_cast<bf16x8*>(dgu + (r + k) * 2 * F + F + c) = pack8(du);
-      }
-  }
+      *reinterpret_cast<bf16x8*>(dgu + (r + k) * 2 * F + c) = pack8(dg);
+      *reinterpret_cast<bf16x8*>(dgu + (r + k) * 2 * F + F + c) = pack8(du);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ embedding
@@ -711,16 +711,20 @@ extern "C" int mt_rope(void* x, const int* pos, const float* inv_ts, long tokens
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-static dim3 gated_grid(long rows, int F) {
-  const long pairs = (rows + 1) / 2;
-  return dim3((unsigned)((F / 8 + 255) / 256), (unsigned)(pairs < 65535 ? pairs : 65535));
+// Threads along a row: its 16-byte columns over as few blocks as 256 threads allow, evenly; what is left of the 256 takes further pairs of rows. (Blocks
+// of 256 columns whatever the width left 62 to 95 % of the threads without work below 768 lanes.)
+static dim3 gated_block(int F) {
+  const int n = F / 8, blocks = (n + 255) / 256, x = (n + blocks - 1) / blocks;
+  return dim3((unsigned)x, (unsigned)(256 / x));
 }
+static unsigned gated_across(int F) { const unsigned x = gated_block(F).x; return (F / 8 + x - 1) / x; }
+static unsigned gated_blocks(long rows, int F) { const long y = 2 * gated_block(F).y; return (unsigned)((rows + y - 1) / y * gated_across(F)); }
 
 extern "C" int mt_gated_act_fwd(const void* gu, void* out, long rows, int F, int code, cudaStream_t st) {
   if (F % 8) return -1;
   if (rows <= 0 || F <= 0) return 0;
   auto k = code == 0 ? gated_act_fwd_kernel<0> : code == 1 ? gated_act_fwd_kernel<1> : code == 2 ? gated_act_fwd_kernel<2> : gated_act_fwd_kernel<3>;
-  k<<<gated_grid(rows, F), 256, 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, F);
+  k<<<gated_blocks(rows, F), gated_block(F), 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, F, gated_across(F));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -728,7 +732,7 @@ extern "C" int mt_gated_act_bwd(const void* dy, const void* gu, void* dgu, long 
   if (F % 8) return -1;
   if (rows <= 0 || F <= 0) return 0;
   auto k = code == 0 ? gated_act_bwd_kernel<0> : code == 1 ? gated_act_bwd_kernel<1> : code == 2 ? gated_act_bwd_kernel<2> : gated_act_bwd_kernel<3>;
-  k<<<gated_grid(rows, F), 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, rows, F);
+  k<<<gated_blocks(rows, F), gated_block(F), 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, rows, F, gated_across(F));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -514,3 +514,23 @@ def test_views_that_start_off_a_16_byte_boundary(at):
     grads.append(torch.autograd.grad(Fn.latent_heads(*leaves, pos, inv, nope, 0.3), leaves, [f(t) for t in up]))
   for w, g in zip(*grads):
     assert torch.equal(w, g)
+
+
+@pytest.mark.parametrize("rows,F", [(1, 16), (77, 96), (515, 512), (33, 768), (130, 1408), (9, 1800), (5, 2056), (3, 14336)])
+def test_gated_act_block_shapes(rows, F):
+  """Widths whose blocks hold one to eight pairs of rows, one or several blocks along a row, ragged last warps and odd row counts: every row the same bits
+  as on its own."""
+  E = _E()
+  gu, dy = (torch.randn(rows, n * F, device="cuda").bfloat16() for n in (2, 1))
+  out, dgu = torch.full_like(dy, 7.0), torch.full_like(gu, 7.0)
+  E.gated_act_fwd(gu, out, 0)
+  E.gated_act_bwd(dy, gu, dgu, 0)
+  x, d = gu.double(), dy.double()
+  g, u, sig = x[:, :F], x[:, F:], torch.sigmoid(x[:, :F])
+  for got, want in ((out, g * sig * u), (dgu[:, F:], d * g * sig), (dgu[:, :F], d * u * sig * (1 + g * (1 - sig)))):
+    assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all())
+  for r in {0, rows // 2, rows - 1}:
+    o1, d1 = torch.empty_like(dy[:1]), torch.empty_like(gu[:1])
+    E.gated_act_fwd(gu[r: r + 1].clone(), o1, 0)
+    E.gated_act_bwd(dy[r: r + 1].clone(), gu[r: r + 1].clone(), d1, 0)
+    assert torch.equal(o1[0], out[r]) and torch.equal(d1[0], dgu[r])
