@@ -268,59 +268,55 @@ def rmsnorm(x: torch.Tensor, p, eps: float, offset: float = 0.0) -> torch.Tensor
 
 class _AddNormFn(torch.autograd.Function):
   """(x + a, norm(x + a)), or (x, norm(x)) without a: the residual stream and what the next sublayer reads. The backward kernel adds the stream's own
-  gradient to the norm's, so that neither pass of the residual add has a kernel of its own."""
+  gradient to the norm's, so that neither pass of the residual add has a kernel of its own. Tensors keep their shape: views as rows are taken inside,
+  where autograd records no node for them (a small model's step waits for the host)."""
 
   @staticmethod
-  def forward(ctx, x2, a2, scale, pv, eps, offset):
-    ctx.pv, ctx.offset, ctx.has_add = pv, offset, a2 is not None
+  def forward(ctx, x, a, scale, pv, eps, offset):
+    ctx.pv, ctx.offset, ctx.has_add = pv, offset, a is not None
     ctx.set_materialize_grads(False)
-    s2, y, rstd = _add_norm_kernel(x2, a2, scale, eps, offset, True)
-    ctx.save_for_backward(s2, scale, rstd)
-    return s2, y
+    s, y, rstd = _add_norm_kernel(x, a, scale, eps, offset, True)
+    ctx.save_for_backward(s, scale, rstd)
+    return s, y
 
   @staticmethod
   def backward(ctx, ds, dy):
     if dy is None:
       return ds, (ds if ctx.has_add else None), None, None, None, None
-    s2, scale, rstd = ctx.saved_tensors
-    pv = ctx.pv
-    dy2 = dy if dy.is_contiguous() else dy.contiguous()
-    if ds is not None and not ds.is_contiguous():
-      ds = ds.contiguous()
-    dx = torch.empty_like(s2)
+    s, scale, rstd = ctx.saved_tensors
+    pv, D = ctx.pv, s.shape[-1]
+    dx = torch.empty_like(s, memory_format=torch.contiguous_format)
     want_ds = pv is not None and pv.main_grad is not None
     if want_ds and not pv.grad_written:
       pv.main_grad.zero_()
       pv.grad_written = True
-    backend.ext().rmsnorm_bwd(dy2, s2, scale, rstd, float(ctx.offset), dx, pv.main_grad if want_ds else None, ds)
+    backend.ext().rmsnorm_bwd(dy.reshape(-1, D).contiguous(), s.reshape(-1, D).contiguous(), scale, rstd, float(ctx.offset), dx.view(-1, D),
+                              pv.main_grad if want_ds else None, None if ds is None else ds.contiguous())
     return dx, (dx if ctx.has_add else None), None, None, None, None
 
 
-def _add_norm_kernel(x2, a2, scale, eps, offset, want_rstd):
-  y = torch.empty_like(x2)
-  s2 = torch.empty_like(x2) if a2 is not None else x2
-  rstd = torch.empty(x2.shape[0], dtype=torch.float32, device=x2.device) if want_rstd else None
-  backend.ext().rmsnorm_fwd(x2, scale, float(eps), float(offset), y, rstd, a2, s2 if a2 is not None else None)
-  return s2, y, rstd
+def _add_norm_kernel(x, a, scale, eps, offset, want_rstd):
+  """x, a of one shape -> (x + a, norm of it) in that shape (a None: x itself, and its norm) and the rows' factors."""
+  D = x.shape[-1]
+  x2 = x.reshape(-1, D).contiguous()
+  y = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+  s = torch.empty_like(y) if a is not None else x
+  rstd = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device) if want_rstd else None
+  backend.ext().rmsnorm_fwd(x2, scale, float(eps), float(offset), y.view(-1, D), rstd, None if a is None else a.contiguous(), None if a is None else s)
+  return s, y, rstd
 
 
 def add_norm(x: torch.Tensor, a, norm):
   """(s, norm(s)) with s = x + a (a None: s = x), for a `layers.blocks.Norm`. Where the stream is bf16 on a GPU and the norm an RMS norm with a scale it is one
   kernel per pass."""
   D = x.shape[-1]
-  if not (getattr(norm, "kind", "") == "rms" and norm.scale is not None and backend.use_cuda_kernels(x) and x.dtype == torch.bfloat16 and D % 8 == 0
+  if not (x.dtype == torch.bfloat16 and backend.use_cuda_kernels(x) and getattr(norm, "kind", "") == "rms" and norm.scale is not None and D % 8 == 0
           and D <= 16384 and norm.scale.shape[-1] == D and (a is None or (a.dtype == x.dtype and a.shape == x.shape))):
     s = x if a is None else x + a
     return s, norm(s)
-  x2 = x.reshape(-1, D)
-  x2 = x2 if x2.is_contiguous() else x2.contiguous()
-  a2 = None if a is None else a.reshape(-1, D)
-  a2 = a2 if a2 is None or a2.is_contiguous() else a2.contiguous()
   if torch.is_grad_enabled():
-    s, y = _AddNormFn.apply(x2, a2, norm.scale.data, norm.scale, norm.eps, norm.offset)
-  else:
-    s, y, _ = _add_norm_kernel(x2, a2, norm.scale.data, norm.eps, norm.offset, False)
-  return s.view(x.shape), y.view(x.shape)
+    return _AddNormFn.apply(x, a, norm.scale.data, norm.scale, norm.eps, norm.offset)
+  return _add_norm_kernel(x, a, norm.scale.data, norm.eps, norm.offset, False)[:2]
 
 
 # =============================================================================== fp32 residual stream

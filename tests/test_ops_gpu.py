@@ -534,3 +534,35 @@ def test_gated_act_block_shapes(rows, F):
     E.gated_act_fwd(gu[r: r + 1].clone(), o1, 0)
     E.gated_act_bwd(dy[r: r + 1].clone(), gu[r: r + 1].clone(), d1, 0)
     assert torch.equal(o1[0], out[r]) and torch.equal(d1[0], dgu[r])
+
+
+def test_add_norm_records_one_node_and_keeps_shapes():
+  """Streams of any shape and stride: one autograd node between the inputs and both results (views as rows would each add one), gradients in the inputs' shapes."""
+  from maxtext_b200.layers.blocks import Constant
+  from maxtext_b200.ops import functional as F
+  D = 264
+
+  class Scale(Constant):
+    shape, main_grad, grad_written = (D,), None, False
+
+  class Norm:
+    kind, eps, offset, scale = "rms", 1e-5, 0.0, Scale((1 + 0.1 * torch.randn(D, device="cuda")).bfloat16())
+  base, a = (torch.randn(3, 5, D, device="cuda").bfloat16() for _ in range(2))
+  up = [torch.randn(3, 5, D, device="cuda").bfloat16() for _ in range(2)]
+  want = None
+  for x0 in (base, base.transpose(0, 1).contiguous().transpose(0, 1)):        # contiguous, and rows of another order in memory
+    for add in (a, None):
+      xs, as_ = x0.detach().requires_grad_(True), a.clone().requires_grad_(True)
+      s, h = F.add_norm(xs, as_ if add is not None else None, Norm)
+      assert s.shape == h.shape == xs.shape
+      assert h.grad_fn is s.grad_fn and "AddNorm" in type(h.grad_fn).__name__
+      assert all(type(f).__name__ == "AccumulateGrad" for f, _ in h.grad_fn.next_functions if f is not None)
+      got = torch.autograd.grad([s, h], [xs] + ([as_] if add is not None else []), up)
+      assert all(t.shape == xs.shape for t in got)
+      if add is None:
+        continue
+      want = want or (s.detach(), h.detach(), got[0])
+      assert torch.equal(s, want[0]) and torch.equal(h, want[1]) and torch.equal(got[0], want[2]) and torch.equal(got[1], want[2])
+      with torch.no_grad():
+        s2, h2 = F.add_norm(xs, as_, Norm)
+      assert torch.equal(s2, want[0]) and torch.equal(h2, want[1])
