@@ -10,7 +10,7 @@ extern "C" {
 int mt_gemm_bf16(const void* a, const void* b, void* c, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int a_mn, int b_mn,
                  int out_f32, int accumulate, int* status, int num_sms, cudaStream_t stream);
 int mt_rmsnorm_fwd(const void* x, const void* add, void* sum, const void* scale, float eps, float offset, void* y, float* rstd, int rows, int D,
-                   cudaStream_t st);
+                   int sms, cudaStream_t st);
 int mt_rmsnorm_bwd(const void* dy, const void* x, const void* scale, const float* rstd, float offset, const void* dres, void* dx, float* dscale,
                    float* partial, int rows, int D, int sms, cudaStream_t st);
 int mt_rmsnorm_bwd_partial_rows(int rows, int D, int sms);
@@ -238,7 +238,7 @@ void rmsnorm_fwd(const torch::Tensor& x, const c10::optional<torch::Tensor>& sca
   c10::optional<Out16> so;
   if (sum) so.emplace(*sum);
   check(mt_rmsnorm_fwd(xa.data_ptr(), aa ? aa->data_ptr() : nullptr, so ? so->ptr() : nullptr, sa ? sa->data_ptr() : nullptr, (float)eps, (float)offset,
-                       ya.ptr(), rstd ? rstd->data_ptr<float>() : nullptr, (int)x.size(0), (int)x.size(1), cur_stream()),
+                       ya.ptr(), rstd ? rstd->data_ptr<float>() : nullptr, (int)x.size(0), (int)x.size(1), num_sms(), cur_stream()),
         "mt_rmsnorm_fwd");
   ya.done();
   if (so) so->done();

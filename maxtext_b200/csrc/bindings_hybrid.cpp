@@ -15,10 +15,10 @@ int mt_ssm_conv(int f32, const void* x, long ldx, const void* w, const void* bia
 int mt_ssm_scan(int f32, const void* x, const void* z, long ldz, const void* q, long ldq, int off, const float* dt, const void* dt_bias, const void* A_log,
                 const void* D, int C, int N, int S, float* rec, const int64_t* slots, const int64_t* lengths, const int64_t* new_lens, void* y, int B,
                 cudaStream_t st);
-int mt_qkv_prep(int f32, const mt::cattn::PrepArgs* a, long N, cudaStream_t st);
+int mt_qkv_prep(int f32, const mt::cattn::PrepArgs* a, long N, int sms, cudaStream_t st);
 int mt_cached_decode(const void* q, const void* k, const void* v, const int64_t* slots, const int64_t* lengths, long max_len, int B, int H, int G, int D, int Dv,
                      float scale, float cap, int window, int chunk, const void* sinks, const void* gate, long ldg, int per_head,
-                     const mt::cattn::DiffArgs* diff, int splits, float* part, float* ml, void* out, cudaStream_t st);
+                     const mt::cattn::DiffArgs* diff, int splits, float* part, float* ml, void* out, int sms, cudaStream_t st);
 int mt_cached_attention(int f32, const void* q, const void* k, const void* v, long max_len, const int64_t* slots, const int64_t* lengths, int B, int S, int H,
                         int G, int D, int Dv, float scale, float cap, int window, int chunk, const void* sinks, void* out, cudaStream_t st);
 int mt_wide_decode(const void* q, const void* k, const void* v, const int64_t* slots, const int64_t* lengths, long max_len, int B, int H, int G, int D, int Dv,
@@ -191,7 +191,7 @@ void qkv_prep(const Tensor& q, const Tensor& k, const Tensor& v, int64_t D, int6
   a.kc = kc.data_ptr(); a.vc = vc.data_ptr(); a.max_len = kc.size(1);
   a.slots = longs(slots, B, "slots"); a.lengths = longs(lengths, B, "lengths"); a.new_lens = longs(new_lens, B, "new_lens");
   c10::cuda::CUDAGuard guard(q.device());
-  done(mt_qkv_prep(f, &a, N, stream()), "qkv_prep");
+  done(mt_qkv_prep(f, &a, N, mt_num_sms(), stream()), "qkv_prep");
 }
 
 // lam: the four lambda vectors of differential attention
@@ -234,7 +234,7 @@ void cached_decode(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
   c10::cuda::CUDAGuard guard(q.device());
   done(mt_cached_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), longs(slots, B, "slots"), longs(lengths, B, "lengths"), k.size(1), (int)B, (int)H, (int)G,
                         (int)D, (int)Dv, (float)scale, (float)cap, (int)window, (int)chunk, sk, gp, gate ? gate->stride(0) : 0, per_head,
-                        lam.empty() ? nullptr : &d, (int)splits, part.data_ptr<float>(), ml.data_ptr<float>(), out.data_ptr(), stream()), "cached_decode", 2);
+                        lam.empty() ? nullptr : &d, (int)splits, part.data_ptr<float>(), ml.data_ptr<float>(), out.data_ptr(), mt_num_sms(), stream()), "cached_decode", 2);
 }
 
 void cached_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& slots, const Tensor& lengths, int64_t S, double scale, double cap,

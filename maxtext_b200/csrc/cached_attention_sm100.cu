@@ -1136,7 +1136,7 @@ head_gate_kernel(const T* __restrict__ o, int dvp, const T* __restrict__ g, long
 }
 
 template <typename T>
-int prep_t(const PrepArgs& a, long N, cudaStream_t st) {
+int prep_t(const PrepArgs& a, long N, int sms, cudaStream_t st) {
   uintptr_t bits = 0;
   for (const void* p : {a.q, a.k, a.v, a.bq, a.bk, a.bv, a.wq, a.wk}) bits |= reinterpret_cast<uintptr_t>(p);
   const bool v4 = a.D % 4 == 0 && a.Dv % 4 == 0 && a.rot % (a.paired ? 4 : 8) == 0 && a.dq % 4 == 0 && a.ldq % 4 == 0 && a.ldk % 4 == 0 && a.ldv % 4 == 0 &&
@@ -1147,7 +1147,7 @@ int prep_t(const PrepArgs& a, long N, cudaStream_t st) {
     if (smem > 40 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
     long parts = 1;
     if (heads_at_once && !a.talk && a.norm != NORM_ALL) {   // a block per pass over the heads, up to about eight blocks per SM
-      const long passes = ((a.H + a.G) * a.maps + heads_at_once - 1) / heads_at_once, room = 8 * 148 / N;
+      const long passes = ((a.H + a.G) * a.maps + heads_at_once - 1) / heads_at_once, room = 8l * sms / N;
       parts = passes < room ? passes : (room < 1 ? 1 : room);
     }
     kernel<<<dim3((unsigned)N, (unsigned)parts), 128, smem, st>>>(a);
@@ -1181,26 +1181,26 @@ int decode_ring(const DecodeArgs& a, int B, cudaStream_t st) {
 // tiles (matrix instructions with two to sixteen rows in use) is what bounds a CTA, and a wave of one, two or three CTAs per SM takes 40, 48 or 72 us at 1500
 // keys (5 : 6 : 9), whichever the number of tiles; so the count of CTAs decides. With two tiles: 360 CTAs 73 us against 93 with three, 2048 CTAs (128 slots, 2048
 // keys) 198 against 214; with three: 480 CTAs 97 us against 114. Other widths keep three tiles.
-bool two_tiles(long ctas) {
-  constexpr long SMS = 148, T[4] = {0, 5, 6, 9};
+bool two_tiles(long ctas, long sms) {
+  constexpr long T[4] = {0, 5, 6, 9};
   auto cost = [&](long per_sm) {
-    const long wave = per_sm * SMS, rest = ctas % wave;
-    return ctas / wave * T[per_sm] + T[(rest + SMS - 1) / SMS];
+    const long wave = per_sm * sms, rest = ctas % wave;
+    return ctas / wave * T[per_sm] + T[(rest + sms - 1) / sms];
   };
   return cost(3) <= cost(2);
 }
 template <int DK, int DVT>
-int decode_run(const DecodeArgs& a, int B, cudaStream_t st) {
+int decode_run(const DecodeArgs& a, int B, int sms, cudaStream_t st) {
   if constexpr (DK == 128 && DVT == 128) {
-    if (two_tiles((long)a.splits * a.G * a.head_blocks * B)) return decode_ring<DK, DVT, 2>(a, B, st);
+    if (two_tiles((long)a.splits * a.G * a.head_blocks * B, sms)) return decode_ring<DK, DVT, 2>(a, B, st);
   }
   return decode_ring<DK, DVT, 3>(a, B, st);
 }
 template <int DK>
-int decode_dv(const DecodeArgs& a, int B, cudaStream_t st) {
-  if (a.Dv <= 64) return decode_run<DK, 64>(a, B, st);
-  if (a.Dv <= 128) return decode_run<DK, 128>(a, B, st);
-  return decode_run<DK, 256>(a, B, st);
+int decode_dv(const DecodeArgs& a, int B, int sms, cudaStream_t st) {
+  if (a.Dv <= 64) return decode_run<DK, 64>(a, B, sms, st);
+  if (a.Dv <= 128) return decode_run<DK, 128>(a, B, sms, st);
+  return decode_run<DK, 256>(a, B, sms, st);
 }
 
 template <typename T>
@@ -1264,20 +1264,20 @@ int gate_t(const void* o, int dvp, const void* g, long ldg, long rows, int HD, i
 using namespace mt::cattn;
 using bf16 = __nv_bfloat16;
 
-extern "C" int mt_qkv_prep(int f32, const PrepArgs* a, long N, cudaStream_t st) {
+extern "C" int mt_qkv_prep(int f32, const PrepArgs* a, long N, int sms, cudaStream_t st) {
   if (N <= 0) return 0;
-  return f32 ? prep_t<float>(*a, N, st) : prep_t<bf16>(*a, N, st);
+  return f32 ? prep_t<float>(*a, N, sms, st) : prep_t<bf16>(*a, N, sms, st);
 }
 
 // diff (or null): q holds two maps per head, H counts both, out is [B, H / 2 * Dv]
 extern "C" int mt_cached_decode(const void* q, const void* k, const void* v, const int64_t* slots, const int64_t* lengths, long max_len, int B, int H, int G,
                                 int D, int Dv, float scale, float cap, int window, int chunk, const void* sinks, const void* gate, long ldg, int per_head,
-                                const DiffArgs* diff, int splits, float* part, float* ml, void* out, cudaStream_t st) {
+                                const DiffArgs* diff, int splits, float* part, float* ml, void* out, int sms, cudaStream_t st) {
   if (B <= 0) return 0;
   if (D % 8 || Dv % 8 || D > 256 || Dv > 256 || H % G || splits < 1 || (diff && (H % 2 || sinks || splits > 64))) return -1;
   DecodeArgs a{(const bf16*)q, (const bf16*)k, (const bf16*)v, slots, lengths, max_len, H, G, D, Dv, window, chunk, splits, (H / G + 15) / 16, scale, cap,
                part, ml};
-  const int rc = D <= 64 ? decode_dv<64>(a, B, st) : (D <= 128 ? decode_dv<128>(a, B, st) : decode_dv<256>(a, B, st));
+  const int rc = D <= 64 ? decode_dv<64>(a, B, sms, st) : (D <= 128 ? decode_dv<128>(a, B, sms, st) : decode_dv<256>(a, B, sms, st));
   if (rc) return rc;
   if (diff)
     diff_merge_kernel<bf16><<<dim3(H / 2, B), 128, 0, st>>>(part, ml, *diff, H / 2, Dv, splits, (const bf16*)gate, ldg, per_head, (bf16*)out);

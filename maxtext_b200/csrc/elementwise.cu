@@ -58,8 +58,10 @@ __device__ __forceinline__ float row_sum(float v, float* smem) {
 // as two kernels (402 + 268 MB) and take 84 us as one (537 MB).
 // Blocks stride over the rows and fetch the next row before they sum the present one: with one row per block, every load waited for a block to start and
 // every store for a barrier (75 us for the plain norm and 117 us for add and norm at 16384 x 4096, 3.6 - 4.6 TB/s; 46 and 84 us now).
+// blocks that share an SM: the kernel is compiled for that many, and the grid counts on them
+constexpr int rms_fwd_resident(int tpr, int vpt, bool add) { return vpt <= 1 ? (tpr == 32 ? 5 : 6) : vpt <= 2 ? 4 : vpt <= 4 || !add ? 2 : 1; }
 template <int TPR, int VPT, bool ADD>
-__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ add,
+__global__ void __launch_bounds__(256, rms_fwd_resident(TPR, VPT, ADD)) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ add,
                                                           __nv_bfloat16* __restrict__ sum, const __nv_bfloat16* __restrict__ scale, float eps, float offset,
                                                           __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out, int rows, int D) {
   __shared__ float red[2][8];
@@ -632,11 +634,11 @@ using namespace mt;
 
 template <int TPR>
 static void launch_rms_fwd(const void* x, const void* add, void* sum, const void* scale, float eps, float offset, void* y, float* rstd, int rows, int D,
-                           cudaStream_t st) {
+                           int sms, cudaStream_t st) {
   const int vpt = (D / 8 + TPR - 1) / TPR;
   const int threads = 256;
   const int rpb = threads / TPR, blocks = (rows + rpb - 1) / rpb;
-  const int most = 148 * (vpt <= 1 ? 6 : vpt <= 2 ? 4 : 2), grid = blocks < most ? blocks : most;   // what is resident at once, so that all blocks have the same rows
+  const int most = sms * rms_fwd_resident(TPR, vpt, add != nullptr), grid = blocks < most ? blocks : most;   // what is resident at once, so that all blocks have the same rows
 #define K(V, A) rmsnorm_fwd_kernel<TPR, V, A><<<grid, threads, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)add, (__nv_bfloat16*)sum, \
                                                                         (const __nv_bfloat16*)scale, eps, offset, (__nv_bfloat16*)y, rstd, rows, D)
 #define L(V) do { if (add) K(V, true); else K(V, false); } while (0)
@@ -647,10 +649,10 @@ static void launch_rms_fwd(const void* x, const void* add, void* sum, const void
 
 // add, sum: both null, or the residual add in front of the norm
 extern "C" int mt_rmsnorm_fwd(const void* x, const void* add, void* sum, const void* scale, float eps, float offset, void* y, float* rstd, int rows,
-                              int D, cudaStream_t st) {
+                              int D, int sms, cudaStream_t st) {
   if (D % 8 || D > 8 * 256 * 8 || !add != !sum) return -1;
-  if (D <= 512) launch_rms_fwd<32>(x, add, sum, scale, eps, offset, y, rstd, rows, D, st);
-  else launch_rms_fwd<256>(x, add, sum, scale, eps, offset, y, rstd, rows, D, st);
+  if (D <= 512) launch_rms_fwd<32>(x, add, sum, scale, eps, offset, y, rstd, rows, D, sms, st);
+  else launch_rms_fwd<256>(x, add, sum, scale, eps, offset, y, rstd, rows, D, sms, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

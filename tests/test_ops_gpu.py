@@ -566,3 +566,26 @@ def test_add_norm_records_one_node_and_keeps_shapes():
       with torch.no_grad():
         s2, h2 = F.add_norm(xs, as_, Norm)
       assert torch.equal(s2, want[0]) and torch.equal(h2, want[1])
+
+
+@pytest.mark.parametrize("rows,D", [(7000, 128), (7000, 512), (2500, 1032), (2500, 4096), (1500, 8192), (1000, 16384)])
+@pytest.mark.parametrize("add", [False, True])
+def test_rows_of_one_block_are_the_same_bits_as_on_their_own(rows, D, add):
+  """More rows than blocks: a block fetches its next row before it sums the present one and takes its two sum buffers in turn. Forward and backward of
+  the first and last rows of a block, of the rows between and of the last ones are the same bits as in a call of few rows, where every block has one."""
+  E = _E()
+  x, a, dy, dres = (torch.randn(rows, D, device="cuda").bfloat16() for _ in range(4))
+  scale = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16()
+
+  def run(x, a, dy, dres):
+    y, s, dx, rstd = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x), torch.empty(x.shape[0], device="cuda")
+    E.rmsnorm_fwd(x, scale, 1e-5, 0.0, y, rstd, a if add else None, s if add else None)
+    E.rmsnorm_bwd(dy, x, scale, rstd, 0.0, dx, None, dres if add else None)
+    return (y, rstd, dx) + ((s,) if add else ())
+  whole = run(x, a, dy, dres)
+  for lo in list(range(0, rows, 140)) + [rows - 3]:
+    cut = slice(lo, min(rows, lo + 140))
+    for w, p in zip(whole, run(*(t[cut].clone() for t in (x, a, dy, dres)))):
+      assert torch.equal(w[cut], p)
+  ref_y = torch.nn.functional.rms_norm((x + a if add else x).double(), (D,), scale.double(), 1e-5)
+  assert bool(((whole[0].double() - ref_y).abs() <= 2 ** -7 * ref_y.abs()).all())
