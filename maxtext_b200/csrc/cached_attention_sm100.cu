@@ -1178,17 +1178,11 @@ int decode_ring(const DecodeArgs& a, int B, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 // Two or three tiles of a warp in shared memory. Heads of 128 lanes let three CTAs share an SM with two tiles, two CTAs with three. A warp's chain of
-// tiles (matrix instructions with two to sixteen rows in use) is what bounds a CTA, and a wave of one, two or three CTAs per SM takes 40, 48 or 72 us at 1500
-// keys (5 : 6 : 9), whichever the number of tiles; so the count of CTAs decides. With two tiles: 360 CTAs 73 us against 93 with three, 2048 CTAs (128 slots, 2048
-// keys) 198 against 214; with three: 480 CTAs 97 us against 114. Other widths keep three tiles.
-bool two_tiles(long ctas, long sms) {
-  constexpr long T[4] = {0, 5, 6, 9};
-  auto cost = [&](long per_sm) {
-    const long wave = per_sm * sms, rest = ctas % wave;
-    return ctas / wave * T[per_sm] + T[(rest + sms - 1) / sms];
-  };
-  return cost(3) <= cost(2);
-}
+// tiles (matrix instructions with two to sixteen rows in use) is what bounds a CTA, so the third CTA is worth more than the third tile (2048 CTAs of 512, 1500
+// keys: 124 us against 134, 269 against 290; 4096 of 2048: 355 against 390) except where it leaves a fourth CTA of every SM to start when three have ended: then two and two
+// are ahead if all sequences are as long (480 CTAs of 512, 1500 keys: 48 against 54 us, 95 against 114; 576 of 8192: 130 against 151; lengths spread by
+// eight: 36 against 32, 73 against 69, 97 against 91). Other widths keep three tiles.
+bool two_tiles(long ctas, long sms) { return ctas <= 3 * sms || ctas > 4 * sms; }
 template <int DK, int DVT>
 int decode_run(const DecodeArgs& a, int B, int sms, cudaStream_t st) {
   if constexpr (DK == 128 && DVT == 128) {
