@@ -17,7 +17,8 @@ struct PrepArgs {
   const float* inv_ts;
   int rot, paired;                     // rotated lanes; paired: neighbouring lanes turn together
   float eps, temp_coef, temp_every;    // temp_every 0: no query temperature
-  int steps;                           // 1: round to the compute type after the bias, each half of the norm and the rotation, as the layers' separate kernels do
+  int steps;                           // 1: round to the compute type after the bias, each half of a norm with weights and the rotation, and take an unweighted
+                                       // norm (NORM_AFTER) of what the rotation stored, as the layers' separate kernels do
   float q_mult;                        // with `steps`: a factor on the queries (rounded again); 1 otherwise
   int S;
   void *qp, *kp, *vp;                  // q [N, H * maps, dq]; k [N, G, dq] and v [N, G, dvp] or null

@@ -157,7 +157,8 @@ qkv_prep_kernel(const PrepArgs a) {
         for (int e = 0; e < VEC; ++e) x[it][e] = 0.f;
       }
     }
-    if (a.norm == NORM_HEAD || a.norm == NORM_AFTER) r = rsqrtf(warp_add(ss) / (float)D + a.eps);   // a rotation leaves the norm as it is
+    const bool late = sizeof(T) == 2 && a.steps && a.norm == NORM_AFTER;       // normalised as rotated and rounded
+    if (a.norm == NORM_HEAD || (a.norm == NORM_AFTER && !late)) r = rsqrtf(warp_add(ss) / (float)D + a.eps);   // a rotation leaves the norm as it is
     // the factor of an element in front of the rotation
     auto scaled = [&](int e0, float (&y)[VEC]) {
       float g[VEC];
@@ -202,10 +203,27 @@ qkv_prep_kernel(const PrepArgs a) {
           x[it][0] = e0 & 1 ? turn_high(y[0], x[it][0], c) : turn_low(x[it][0], y[0], c);
         }
       }
-      if (!key) {
+    }
+    if (late) {
+      ss = 0.f;
+#pragma unroll
+      for (int it = 0; it < ITER; ++it)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {                      // lanes beyond D hold zeros
+          x[it][e] = stored<T>(x[it][e]);
+          ss += x[it][e] * x[it][e];
+        }
+      r = rsqrtf(warp_add(ss) / (float)D + a.eps);
+#pragma unroll
+      for (int it = 0; it < ITER; ++it)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) x[it][e] *= r;
+    }
+    if (!key) {
+#pragma unroll
+      for (int it = 0; it < ITER; ++it)
 #pragma unroll
         for (int e = 0; e < VEC; ++e) x[it][e] = (a.steps ? stored<T>(stored<T>(x[it][e]) * a.q_mult) : x[it][e]) * warm;
-      }
     }
     const int m = head % a.maps;                            // this map's lanes of the head
     T* dst = key ? (a.kp ? static_cast<T*>(a.kp) + (n * a.G + head / a.maps) * (TALK ? D : a.dq) : nullptr) : static_cast<T*>(a.qp) + (n * HM + head) * a.dq;
@@ -344,14 +362,16 @@ qkv_prep_wide_kernel(const PrepArgs a) {
     float next[VEC];
     raw(h + STEP, next);
     float r = key ? rstd_k : rstd_q;
-    if (a.norm == NORM_HEAD || a.norm == NORM_AFTER) {      // a rotation leaves the norm as it is
+    const bool late = sizeof(T) == 2 && a.steps && a.norm == NORM_AFTER;      // normalised as rotated and rounded
+    auto rstd_of_head = [&] {
       float ss = 0.f;
 #pragma unroll
       for (int e = 0; e < VEC; ++e) ss += x[e] * x[e];
 #pragma unroll
       for (int w = LPH / 2; w > 0; w >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, w);
-      r = rsqrtf(ss / (float)D + a.eps);
-    }
+      return rsqrtf(ss / (float)D + a.eps);
+    };
+    if (a.norm == NORM_HEAD || (a.norm == NORM_AFTER && !late)) r = rstd_of_head();           // a rotation leaves the norm as it is
     if (a.norm >= NORM_HEAD && live) {
       float g[VEC];
       load_vec<VEC>(static_cast<const T*>(key ? a.wk : a.wq) + (a.norm == NORM_ALL ? (long)head * D : 0) + e0, g);
@@ -382,6 +402,13 @@ qkv_prep_wide_kernel(const PrepArgs a) {
           x[e] = low ? turn_low(x[e], y, c) : turn_high(y, x[e], c);
         }
       }
+    }
+    if (late) {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) x[e] = stored<T>(x[e]);
+      r = rstd_of_head();
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) x[e] *= r;
     }
     const int m = head % a.maps;                            // this map's lanes of the head
     if (live) {

@@ -139,7 +139,8 @@ def serve(layer, q, k, v, g, ctx):
   kp = torch.empty(N, G, dq, dtype=q.dtype, device=q.device) if pack_k else None
   copy_v = pack_k and (dvp != Dv or bias[2] is not None or v.stride(0) % 8 != 0 or v.data_ptr() % 16 != 0)
   vp = torch.empty(N, G, dvp, dtype=q.dtype, device=q.device) if copy_v else None
-  # plain layers keep the roundings of their separate kernels: a prompt's keys are the same whichever path wrote them
+  # plain layers round where their separate kernels do, so a prompt's keys are the same whichever path wrote them. (Where a norm's sum of squares runs in another
+  # order there, one over all heads, an unweighted one or of heads that are no multiple of 8 wide, its factor may differ by an ulp of fp32.)
   steps = layer.sizes is None
   E.qkv_prep(q, k, v, D, Dv, ctx.positions.contiguous(), layer.inv_ts if rot else None, rot, eps, qp, kp, vp, cache.k, cache.v, cache.slot_ids,
              cache.lengths, cache.new_lens, *bias, *norms, layer.interleaved, maps, *temp, steps=steps, q_mult=scale if steps else 1.0)

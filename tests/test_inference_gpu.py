@@ -149,3 +149,71 @@ def test_decode_attention_is_the_same_bits_however_many_ctas_share_an_sm():
   s = torch.softmax(torch.einsum("gjd,ngd->gjn", q[b].view(G, 2, D).double(), k[b, :n].double()) * 0.1, -1)
   want = torch.einsum("gjn,ngd->gjd", s, v[b, :n].double()).reshape(-1)
   assert bool(((few[b].double() - want).abs() <= 2 ** -7 * want.abs().max()).all())
+
+
+@pytest.mark.parametrize("D,rot", [(16, 16), (20, 16), (64, 32), (128, 128), (200, 64), (320, 320)])
+@pytest.mark.parametrize("paired", [False, True])
+def test_unweighted_norm_of_rotated_heads_rounds_like_the_separate_steps(D, rot, paired):
+  """Rotated, rounded, normalised by the rounded row, rounded, then the factor and the temperature on the queries, each rounded. Only the sum of squares runs in
+  another order, which moves a factor by an ulp of fp32: fewer than one element in 200 rounds to the other bf16 neighbour."""
+  from maxtext_b200.ops import backend
+  from maxtext_b200.ops import reference as ref
+  E = backend.ext(required=True)
+  g = torch.Generator(device="cuda").manual_seed(D)
+  B, S, H, G, L = 3, 7, 4, 2, 40
+  N, eps, mult, coef, every = B * S, 1e-5, 0.3, 0.1, 8.0
+  q, k, v = ((torch.randn(N, n * D, device="cuda", generator=g) * 3).bfloat16() for n in (H, G, G))
+  lengths = torch.tensor([5, 0, 20], device="cuda")
+  pos = (lengths[:, None] + torch.arange(S, device="cuda")).reshape(-1)
+  inv = ref.rope_inv_timescale(rot, 1, 10000).cuda()
+  qp = torch.empty(N, H, D, device="cuda", dtype=torch.bfloat16)
+  kc, vc = torch.zeros(B, L, G, D, device="cuda", dtype=torch.bfloat16), torch.zeros(B, L, G, D, device="cuda", dtype=torch.bfloat16)
+  E.qkv_prep(q, k, v, D, D, pos, inv, rot, eps, qp, None, None, kc, vc, torch.arange(B, device="cuda"), lengths, None, paired=paired, temp_coef=coef,
+             temp_every=every, steps=True, q_mult=mult)
+
+  def steps(t, n):
+    t = t.view(N, n, D).clone()
+    E.rope_inplace(t, pos.to(torch.int32), inv, n, paired, False, rot)
+    f = t.float()
+    return (f * torch.rsqrt(f.pow(2).mean(-1, keepdim=True) + eps)).bfloat16()
+  wk = steps(k, G)
+  wq = steps(q, H) * mult
+  wq = (wq.float() * (torch.log(torch.floor((pos.float() + 1) / every) + 1) * coef + 1)[:, None, None]).bfloat16()
+  gk = torch.cat([kc[b, int(lengths[b]): int(lengths[b]) + S] for b in range(B)])
+  for got, want in ((gk, wk), (qp, wq)):
+    assert float((got != want).float().mean()) <= 1 / 200
+    assert bool(((got.float() - want.float()).abs() <= 2 ** -7 * want.float().abs() + 1e-6).all())
+  assert torch.equal(torch.cat([vc[b, int(lengths[b]): int(lengths[b]) + S] for b in range(B)]).reshape(N, -1), v)
+
+
+@pytest.mark.parametrize("name", ["llama3-8b", "gemma2-2b", "gemma3-4b", "qwen3-8b", "qwen2.5-7b", "olmo3-7b", "llama4-17b-16e", "gpt-oss-20b"])
+@pytest.mark.parametrize("head_dim", [16, 20, 128])
+def test_cached_keys_of_the_first_layer_are_the_same_whichever_path_wrote_them(name, head_dim, monkeypatch):
+  """Both paths read the same projections of the first layer. Where no norm follows, or one per head whose sum both take in the same order (widths in multiples
+  of 8), the cached keys are the same bits; elsewhere the sum of squares (or, with biases, the product's) runs in another order, and fewer than one element
+  in 200 rounds to the other neighbour. Queries show in the logits."""
+  from helpers import tiny_config
+  from maxtext_b200.inference.maxengine import MaxEngine
+  from maxtext_b200.layers.blocks import Attention
+  more = [f"head_dim={head_dim}", "max_target_length=48", "max_prefill_predict_length=40", "per_device_batch_size=3", "weight_init=normal",
+          "dtype=bfloat16", "hardware=gpu"]
+  g = torch.Generator().manual_seed(2)
+  prompts = [torch.randint(1, 256, (n,), generator=g).tolist() for n in (30, 17, 40)]
+  real, kept = Attention.serves, []
+  for served in (False, True):
+    used = []
+    monkeypatch.setattr(Attention, "serves", lambda self, x, ctx: used.append(served and real(self, x, ctx)) or used[-1])
+    eng = MaxEngine(tiny_config(name, extra=more), device="cuda")
+    eng.load_params(seed=3)
+    state = eng.init_decode_state(3)
+    eng.extend(state, [0, 1, 2], prompts)
+    assert any(used) == served
+    c = state.caches[0][0]
+    kept.append([torch.cat([getattr(c, n)[b, : len(p)] for b, p in enumerate(prompts)]) for n in ("k", "v")])
+  (k0, v0), (k1, v1) = kept
+  exact = name in ("llama3-8b", "gemma2-2b") or (name in ("gemma3-4b", "qwen3-8b") and head_dim % 8 == 0)
+  for a, b in ((k0, k1), (v0, v1)):
+    if exact:
+      assert torch.equal(a, b)
+    assert float((a != b).float().mean()) <= 1 / 200
+    assert bool(((a.float() - b.float()).abs() <= 2 ** -7 * a.float().abs() + 2 ** -9 * a.float().abs().max()).all())
