@@ -156,8 +156,8 @@ def serve(layer, q, k, v, g, ctx):
     return _gate(o.reshape(N, H * maps, dvp), g, H, Dv, layer)
   if widths is None:
     return plain(qp, cache, S, scale, cap, win, sinks, g, chunk, layer)
-  # normalised q and k bound every score by D * scale
-  mode = F.CAP_SMALL if layer.l2_qk_norm and D * abs(scale) <= 0.3 * cap else F.CAP_EXACT
+  # normalised q and k bound every score by D * scale (plain layers hold the factor in their queries, and cap as `attend` does)
+  mode = F.CAP_SMALL if layer.l2_qk_norm and not steps and D * abs(scale) <= 0.3 * cap else F.CAP_EXACT
   if fresh:
     o = _flash(qp.view(B, S, H * maps, dq), kp.view(B, S, G, dq), vp.view(B, S, G, dvp) if vp is not None else _rows(v, B, S, G, Dv), ctx.positions,
                ctx.segment_ids, scale, cap, win, sinks, mode, chunk=chunk)

@@ -217,3 +217,31 @@ def test_cached_keys_of_the_first_layer_are_the_same_whichever_path_wrote_them(n
       assert torch.equal(a, b)
     assert float((a != b).float().mean()) <= 1 / 200
     assert bool(((a.float() - b.float()).abs() <= 2 ** -7 * a.float().abs() + 2 ** -9 * a.float().abs().max()).all())
+
+
+def test_soft_cap_behind_normalised_heads_is_exact_for_plain_layers(monkeypatch):
+  """The kernel's short form of the cap holds for scores up to 0.3 of it. A plain layer's factor is part of its queries by then, so the width alone bounds nothing:
+  with a factor of 4 the scores of 16 normalised lanes reach 64 under a cap of 60."""
+  from helpers import tiny_config
+  from maxtext_b200.inference.maxengine import MaxEngine
+  from maxtext_b200.layers.blocks import Attention
+  from maxtext_b200.ops import cached_attention as CA
+  from maxtext_b200.ops import functional as F
+  cfg = tiny_config("llama4-17b-16e", extra=["head_dim=16", "max_target_length=48", "max_prefill_predict_length=40", "per_device_batch_size=1",
+                                             "weight_init=normal", "dtype=bfloat16", "hardware=gpu"])
+  eng = MaxEngine(cfg, device="cuda")
+  eng.load_params(seed=3)
+  attns = [b.attn for layer in eng.model.runs for b in layer.blocks]
+  assert any(a.l2_qk_norm for a in attns)
+  for a in attns:
+    a.soft_cap, a.query_scalar = 60.0, 4.0
+  modes, real, serves = [], CA._flash, Attention.serves
+  monkeypatch.setattr(CA, "_flash", lambda *a, **kw: modes.append(a[9]) or real(*a, **kw))
+  g = torch.Generator().manual_seed(4)
+  prompt = torch.randint(1, 256, (30,), generator=g).tolist()
+  out = []
+  for served in (False, True):
+    monkeypatch.setattr(Attention, "serves", lambda self, x, ctx, s=served: s and serves(self, x, ctx))
+    out.append(eng.extend(eng.init_decode_state(1), [0], [prompt]).float())
+  assert modes and all(m == F.CAP_EXACT for m in modes)
+  assert float((out[0] - out[1]).norm() / out[0].norm()) <= 2 ** -5
