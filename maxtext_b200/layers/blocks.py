@@ -482,7 +482,9 @@ class Attention:
     from ..ops import cached_attention as CA
     B, S, _ = x.shape
     if rows is None:
-      if self.qkvg is not None and self.qkvg.fusable():
+      # plain layers with biases have 8-bit scales per projection (`_project`), not one for all of them
+      apart = self.sizes is None and self.bq is not None and F._quant.mode() != ""
+      if self.qkvg is not None and not apart and self.qkvg.fusable():
         rows = torch.split(F.linear(x, self.qkvg).view(B * S, -1), self.qkvg.rows, dim=-1)
       else:
         rows = [F.linear(x, w).view(B * S, -1) for w in self.in_parts]

@@ -245,3 +245,34 @@ def test_soft_cap_behind_normalised_heads_is_exact_for_plain_layers(monkeypatch)
     out.append(eng.extend(eng.init_decode_state(1), [0], [prompt]).float())
   assert modes and all(m == F.CAP_EXACT for m in modes)
   assert float((out[0] - out[1]).norm() / out[0].norm()) <= 2 ** -5
+
+
+def test_served_projections_with_biases_keep_their_8_bit_scales(monkeypatch):
+  """8-bit products scale a weight by its largest element. Projections with biases are products of their own, each with its scale, whichever path serves them:
+  with queries' weights far larger than the keys', one scale for all of them would round the keys' differently."""
+  from helpers import tiny_config
+  from maxtext_b200.inference.maxengine import MaxEngine
+  from maxtext_b200.layers.blocks import Attention
+  from maxtext_b200.ops import quantization as Q
+  cfg = tiny_config("qwen2.5-7b", extra=["base_emb_dim=128", "base_mlp_dim=256", "head_dim=64", "max_target_length=160", "max_prefill_predict_length=140",
+                                         "per_device_batch_size=1", "weight_init=normal", "dtype=bfloat16", "hardware=gpu"])
+  eng = MaxEngine(cfg, device="cuda")
+  eng.load_params(seed=3)
+  for layer in eng.model.runs:
+    layer.blocks[0].attn.q.data.mul_(37.0)
+  g = torch.Generator().manual_seed(4)
+  prompt = torch.randint(1, 256, (128,), generator=g).tolist()
+  serves, kept = Attention.serves, []
+  Q.set_mode("fp8")
+  try:
+    for served in (False, True):
+      used = []
+      monkeypatch.setattr(Attention, "serves", lambda self, x, ctx: used.append(served and serves(self, x, ctx)) or used[-1])
+      state = eng.init_decode_state(1)
+      eng.extend(state, [0], [prompt])
+      assert any(used) == served
+      kept.append([getattr(state.caches[0][0], n)[0, :128].clone() for n in ("k", "v")])
+  finally:
+    Q.set_mode("")
+  for a, b in zip(*kept):
+    assert torch.equal(a, b)
