@@ -50,9 +50,16 @@ def _small_m_wins(M, N, K) -> bool:
   return M <= 32 and N <= 4096 and K <= 4096
 
 
-def _gemm_supported(M, N, K, a, b, k_strided=False):
-  """`k_strided`: the summed dimension is the slow one of both operands (a weight gradient), so that its length needs no alignment."""
-  return a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and (k_strided or K % 8 == 0) and N % 8 == 0 and K >= 16
+def _gemm_supported(M, N, K, a, b, any_k=False):
+  return a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and (any_k or K % 8 == 0) and N % 8 == 0 and K >= 16
+
+
+def _any_k(M, N, ta, tb, accumulate) -> bool:
+  """Does a product of a K that is no multiple of 8 run on the tcgen05 kernel? It can where K is the slow dimension of both operands (a weight gradient over
+  any number of tokens). A first gradient stays with the library, which writes fp32 and splits K (2048 x 2048 over 16383 tokens: 92 us against 96;
+  512 x 512: 29 against 88). One that adds to another would come out of it in bf16 and be added by a second kernel, so from 2048 x 2048 on, where the output
+  has a tile for nearly every SM, it runs here; below, the library is ahead even so (1408 x 2048 over 16383: 81 against 92 us; 512 x 512: 38 against 88)."""
+  return ta and not tb and accumulate and M * N >= 1 << 22
 
 
 def mm(a: torch.Tensor, b: torch.Tensor, ta: bool, tb: bool, out: torch.Tensor | None = None,
@@ -74,7 +81,7 @@ def mm(a: torch.Tensor, b: torch.Tensor, ta: bool, tb: bool, out: torch.Tensor |
         and E.gemm_small_m_supported(a, b, out)):
       E.gemm_small_m(a, b, out)            # decode-sized products stream the weight once (csrc/gemm_small_m.cu)
       return out
-    if _GEMM_IMPL == "tcgen05" and _gemm_supported(M, N, K, a, b, ta and not tb) and E.gemm_supported(a, b, out, ta, tb):
+    if _GEMM_IMPL == "tcgen05" and _gemm_supported(M, N, K, a, b, _any_k(M, N, ta, tb, accumulate)) and E.gemm_supported(a, b, out, ta, tb):
       E.gemm(a, b, out, ta, tb, accumulate)
       return out
     if _GEMM_IMPL == "tcgen05":

@@ -161,3 +161,21 @@ def test_gemm_one_wave_of_narrow_tiles(M, N, K):
     E.gemm(a, b, x, False, True, False)
     E.gemm_pair(a, b, y, False, True, False)
     assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("M,N,K,accumulate,own", [(512, 512, 333, False, False), (512, 512, 333, True, False), (2048, 2048, 333, False, False),
+                                                  (2048, 2048, 333, True, True), (2048, 2040, 333, True, False), (512, 512, 336, True, True)])
+def test_weight_gradients_over_odd_counts_go_where_they_are_faster(M, N, K, accumulate, own):
+  """The library for first gradients and small outputs over a K that is no multiple of 8, the framework's kernel for sums into a large output. The library's
+  sum comes as bf16 (2**-9 of itself) before it is added."""
+  from maxtext_b200.ops import functional as F
+  a, b = torch.randn(K, M, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+  start = torch.randn(M, N, device="cuda")
+  out = start.clone()
+  before = F._GEMM_FALLBACKS
+  F.mm(a, b, True, False, out, accumulate)
+  assert F._GEMM_FALLBACKS - before == (0 if own else 1)
+  prod = a.double().t() @ b.double()
+  want = prod + (start.double() if accumulate else 0)
+  bound = 2.0 ** -16 * K ** 0.5 * 8 + (2.0 ** -8 * prod.abs() if accumulate and not own else 0)
+  assert bool(((out.double() - want).abs() <= bound + 2.0 ** -22 * want.abs()).all())
