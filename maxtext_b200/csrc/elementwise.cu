@@ -55,9 +55,9 @@ __device__ __forceinline__ float row_sum(float v, float* smem) {
 // ------------------------------------------------------------------------------------------------ RMSNorm forward
 // y = bf16(x * rstd) * bf16(scale + offset), both roundings as in the reference layer. With `add` the row is bf16(x + add), which also goes to
 // `sum`: the residual add in front of a norm, in the norm's own pass. Bandwidth-bound; at 16384 rows of 4096 lanes the add and the norm took 65 + 85 us
-// as two kernels (402 + 268 MB) and take 84 us as one (537 MB).
+// as two kernels (402 + 268 MB) and take 90 us as one (537 MB).
 // Blocks stride over the rows and fetch the next row before they sum the present one: with one row per block, every load waited for a block to start and
-// every store for a barrier (75 us for the plain norm and 117 us for add and norm at 16384 x 4096, 3.6 - 4.6 TB/s; 46 and 84 us now).
+// every store for a barrier (75 us for the plain norm and 117 us for add and norm at 16384 x 4096, 3.6 - 4.6 TB/s; 46 and 90 us now).
 // blocks that share an SM: the kernel is compiled for that many, and the grid counts on them
 constexpr int rms_fwd_resident(int tpr, int vpt, bool add) { return vpt <= 1 ? (tpr == 32 ? 5 : 6) : vpt <= 2 ? 4 : vpt <= 4 || !add ? 2 : 1; }
 template <int TPR, int VPT, bool ADD>
@@ -145,7 +145,8 @@ __global__ void __launch_bounds__(256, rms_fwd_resident(TPR, VPT, ADD)) rmsnorm_
 // is the same bits as of a norm and an add on their own.
 // Blocks stride over rows and keep per-column dscale partials in registers; each (block, row slot) writes its partial row into `partial`, and
 // rms_dscale_reduce_kernel adds the rows up in a fixed order: no atomics, so the result is bitwise reproducible.
-// As in the forward pass the next row is fetched before the present one is summed: 110 us for 16384 x 4096 with a stream gradient (537 MB), 192 us without.
+// As in the forward pass the next row is fetched before the present one is summed: 110 us for 16384 x 4096 with a stream gradient and a scale's (537 MB), of
+// which the reduction below is 6, 192 us without.
 template <int TPR, int VPT>
 __global__ void __launch_bounds__(256, TPR == 32 ? (VPT == 1 ? 4 : 1) : VPT == 1 ? 3 : VPT == 2 ? 2 : 1) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                    const __nv_bfloat16* __restrict__ scale, const float* __restrict__ rstd_in, float offset,
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(256, TPR == 32 ? (VPT == 1 ? 4 : 1) : VPT == 1
 // pairs. The four serial chains per column are what bounds it, so nothing else may wait in them: a block of 256 threads fetches 16 KB of its COLS columns ahead,
 // and a thread per column and sum adds up the rows that wait in shared memory. Narrow widths have more blocks with eight columns (32-byte pieces); from 1024
 // columns on there are enough with 32. A thread per column that loads what it adds (16 - 32 blocks at the usual widths) took 47 us for 592 rows of 4096
-// columns and 95 us for the 4736 rows of a 128-wide head norm; the whole backward pass takes 60 and 22 us at these sizes now (8192 x 4096, 4800 x 128).
+// columns and 95 us for the 4736 rows of a 128-wide head norm; 6.4 and 11 us now.
 template <int COLS>
 __global__ void __launch_bounds__(256) rms_dscale_reduce_kernel(const float* __restrict__ partial, int nrows, int D, float* __restrict__ dscale) {
   constexpr int ROWS = 4096 / COLS, V = COLS / 4, STEP = 256 / V, PER = ROWS / STEP;      // V 16-byte pieces per row, PER of a thread per tile
