@@ -411,13 +411,12 @@ __device__ __forceinline__ float act_grad(float g, int code) {
 
 // gu [rows, 2F] = [gate | up] -> out [rows, F]. Bandwidth-bound: a thread takes a 16-byte column of two rows at a time, so that it has four (backward: six)
 // loads in flight and no index to divide; a block is as wide as the row needs (gated_block) and takes several pairs of rows where that is less than 256
-// threads. One vector per thread out of a flat index with 64-bit divisions took 283 us forward and 482 us backward for 16384 x 14336 and 51 and 80 us for
-// 24576 x 1408; 246, 371, 47 and 70 us here (5.7 TB/s). The division of the sigmoid is what keeps the forward pass from copy rate.
+// threads. One vector per thread out of a flat index with 64-bit divisions took 281 us forward and 479 us backward for 16384 x 14336 and 51 and 80 us for
+// 24576 x 1408; 217, 360, 43 and 68 us here (6.5 TB/s). A division of the block's index for its row and column cost 30 and 10 us at the first size.
 template <int CODE>
-__global__ void __launch_bounds__(256) gated_act_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long rows, int F,
-                                                            unsigned across) {
-  const int c = (blockIdx.x % across * blockDim.x + threadIdx.x) * 8;
-  const long r = (blockIdx.x / across * (long)blockDim.y + threadIdx.y) * 2;
+__global__ void __launch_bounds__(256) gated_act_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long rows, int F) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  const long r = ((blockIdx.z * (long)gridDim.y + blockIdx.y) * blockDim.y + threadIdx.y) * 2;
   if (c >= F) return;
   bf16x8 g[2], u[2];
 #pragma unroll
@@ -440,9 +439,9 @@ __global__ void __launch_bounds__(256) gated_act_fwd_kernel(const __nv_bfloat16*
 
 template <int CODE>
 __global__ void __launch_bounds__(256, 5) gated_act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gu,
-                                                            __nv_bfloat16* __restrict__ dgu, long rows, int F, unsigned across) {
-  const int c = (blockIdx.x % across * blockDim.x + threadIdx.x) * 8;
-  const long r = (blockIdx.x / across * (long)blockDim.y + threadIdx.y) * 2;
+                                                            __nv_bfloat16* __restrict__ dgu, long rows, int F) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  const long r = ((blockIdx.z * (long)gridDim.y + blockIdx.y) * blockDim.y + threadIdx.y) * 2;
   if (c >= F) return;
   bf16x8 g[2], u[2], d[2];
 #pragma unroll
@@ -722,14 +721,17 @@ static dim3 gated_block(int F) {
   const int n = F / 8, blocks = (n + 255) / 256, x = (n + blocks - 1) / blocks;
   return dim3((unsigned)x, (unsigned)(256 / x));
 }
-static unsigned gated_across(int F) { const unsigned x = gated_block(F).x; return (F / 8 + x - 1) / x; }
-static unsigned gated_blocks(long rows, int F) { const long y = 2 * gated_block(F).y; return (unsigned)((rows + y - 1) / y * gated_across(F)); }
+static dim3 gated_grid(long rows, int F) {       // y and z count the groups of rows: y alone ends at 65535
+  const dim3 b = gated_block(F);
+  const long groups = (rows + 2 * b.y - 1) / (2 * b.y), z = (groups + 65534) / 65535;
+  return dim3((F / 8 + b.x - 1) / b.x, (unsigned)((groups + z - 1) / z), (unsigned)z);
+}
 
 extern "C" int mt_gated_act_fwd(const void* gu, void* out, long rows, int F, int code, cudaStream_t st) {
   if (F % 8) return -1;
   if (rows <= 0 || F <= 0) return 0;
   auto k = code == 0 ? gated_act_fwd_kernel<0> : code == 1 ? gated_act_fwd_kernel<1> : code == 2 ? gated_act_fwd_kernel<2> : gated_act_fwd_kernel<3>;
-  k<<<gated_blocks(rows, F), gated_block(F), 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, F, gated_across(F));
+  k<<<gated_grid(rows, F), gated_block(F), 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)out, rows, F);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -737,7 +739,7 @@ extern "C" int mt_gated_act_bwd(const void* dy, const void* gu, void* dgu, long 
   if (F % 8) return -1;
   if (rows <= 0 || F <= 0) return 0;
   auto k = code == 0 ? gated_act_bwd_kernel<0> : code == 1 ? gated_act_bwd_kernel<1> : code == 2 ? gated_act_bwd_kernel<2> : gated_act_bwd_kernel<3>;
-  k<<<gated_blocks(rows, F), gated_block(F), 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, rows, F, gated_across(F));
+  k<<<gated_grid(rows, F), gated_block(F), 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, rows, F);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -591,3 +591,18 @@ def test_rows_of_one_block_are_the_same_bits_as_on_their_own(rows, D, add):
       assert torch.equal(w[cut], p)
   ref_y = torch.nn.functional.rms_norm((x + a if add else x).double(), (D,), scale.double(), 1e-5)
   assert bool(((whole[0].double() - ref_y).abs() <= 2 ** -7 * ref_y.abs()).all())
+
+
+def test_gated_act_over_more_rows_than_one_grid_axis():
+  """Narrow rows by the million: groups of row pairs beyond 65535 go on along the grid's third axis."""
+  E = _E()
+  rows, F = 65535 * 2 * 21 * 2 + 77, 96                        # 21 pairs of rows per block: a bit more than two times the axis
+  gu = torch.randn(1, 2 * F, device="cuda").bfloat16().expand(rows, -1).contiguous()
+  dy = torch.randn(1, F, device="cuda").bfloat16().expand(rows, -1).contiguous()
+  out, dgu = torch.full_like(dy, 7.0), torch.full_like(gu, 7.0)
+  E.gated_act_fwd(gu, out, 0)
+  E.gated_act_bwd(dy, gu, dgu, 0)
+  one, done = torch.empty_like(dy[:1]), torch.empty_like(gu[:1])
+  E.gated_act_fwd(gu[:1], one, 0)
+  E.gated_act_bwd(dy[:1], gu[:1], done, 0)
+  assert bool((out == one).all()) and bool((dgu == done).all())
